@@ -177,9 +177,15 @@ int hbsa_block_decisions(const hbsa_forward_args* args, uint8_t* decisions, int3
   return 0;
 }
 
+static size_t backward_bytes(int64_t total_q, int64_t total_k, int nhead_q, int nhead_k, int headdim) {
+  const size_t generic = hbsa::backward_workspace_bytes(total_q, total_k, nhead_q, nhead_k, headdim);
+  const size_t sm100 = hbsa::backward_sm100_workspace_bytes(total_q, nhead_q);
+  return generic > sm100 ? generic : sm100;        // the dtype and the strides that decide between the two are not known here
+}
+
 size_t hbsa_backward_workspace_bytes(int64_t total_q, int64_t total_k, int nhead_q, int nhead_k, int headdim) {
   if (total_q < 0 || total_k < 0 || nhead_q <= 0 || nhead_k <= 0 || headdim <= 0) return 0;
-  return hbsa::backward_workspace_bytes(total_q, total_k, nhead_q, nhead_k, headdim);
+  return backward_bytes(total_q, total_k, nhead_q, nhead_k, headdim);
 }
 
 int hbsa_backward(const hbsa_backward_args* b, void* stream_) {
@@ -190,13 +196,25 @@ int hbsa_backward(const hbsa_backward_args* b, void* stream_) {
   if (rc != 0) return rc;
   if (!b->d_o || !b->dq || !b->dk || !b->dv || !b->grad_workspace) return fail(HBSA_ERR_NULL, "d_o, dq, dk, dv and grad_workspace must not be NULL");
   if (!b->fwd.lse) return fail(HBSA_ERR_NULL, "the backward needs the lse of the forward (hbsa_forward_args.lse)");
-  if (b->grad_workspace_bytes < hbsa::backward_workspace_bytes(b->fwd.total_q, b->fwd.total_k, b->fwd.nhead_q, b->fwd.nhead_k, b->fwd.headdim))
+  if (b->grad_workspace_bytes < backward_bytes(b->fwd.total_q, b->fwd.total_k, b->fwd.nhead_q, b->fwd.nhead_k, b->fwd.headdim))
     return fail(HBSA_ERR_WORKSPACE, "grad_workspace is smaller than hbsa_backward_workspace_bytes()");
   if (((uintptr_t)b->grad_workspace) % 256 != 0) return fail(HBSA_ERR_WORKSPACE, "grad_workspace must be 256-byte aligned");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   hbsa::Workspace ws = hbsa::make_workspace(b->fwd.workspace, p.nhead_k, p.num_q_block, p.num_k_block, p.batch);
+  const char* why = hbsa::backward_sm100_ineligible_reason(*b, p.scale);
+  if (b->fwd.impl == HBSA_IMPL_SM100 && why) {
+    snprintf(g_err, sizeof(g_err), "the tcgen05 backward cannot run this problem: %s", why);
+    return HBSA_ERR_UNSUPPORTED;
+  }
+  const bool sm100 = !why && b->fwd.impl != HBSA_IMPL_GENERIC;
+  if (sm100) p.kv_tile = hbsa::backward_sm100_kv_tile_rows(p.kbs);
   cudaError_t e = hbsa::launch_schedule(p, ws, nullptr, stream);
   if (e != cudaSuccess) return fail_cuda(e, "hbsa_backward (schedule)");
+  if (sm100) {
+    const char* text = "";
+    rc = hbsa::launch_backward_sm100(p, ws, *b, stream, &text);
+    return rc != 0 ? fail(rc, text) : 0;
+  }
   e = hbsa::launch_backward_generic(p, ws, *b, stream);
   return e == cudaSuccess ? 0 : fail_cuda(e, "hbsa_backward");
 }

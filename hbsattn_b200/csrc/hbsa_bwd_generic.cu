@@ -1,4 +1,5 @@
-// Backward of the block-sparse attention forward on the CUDA cores: dQ, dK, dV over the active block pairs.
+// Backward of the block-sparse attention forward on the CUDA cores: dQ, dK, dV over the active block pairs, for what the
+// tensor-core backward (hbsa_bwd_sm100.cu) does not take: fp32, head dimensions above 128, odd strides.
 //
 // The reference has no backward (hbsattn/hbsa_interface.py:30-32 raises NotImplementedError; its README lists it
 // as future work), so there is nothing to be compatible with except the mathematics of the forward it does have

@@ -1,0 +1,878 @@
+// Backward of the block-sparse attention on the 5th-generation tensor cores (tcgen05 + TMEM + TMA), bf16 / fp16,
+// head dimensions up to 128.  The mathematics is that of hbsa_bwd_generic.cu:
+//     P = exp(scale * Q K^T - lse)      delta = rowsum(dO * O)      dS = P * (dO V^T - delta)
+//     dV = P^T dO                       dQ = scale * dS K           dK = scale * dS^T Q
+//
+// One kernel template, launched twice, each time with one operand pair stationary and the other streamed past it:
+//   dK/dV (KV = true):  K, V of up to 128 keys of one k-block stay; Q, dO of the q-blocks that attend to it are streamed in
+//                       tiles of at most 64 rows (tokens x GQA heads).  S^T = K Q^T and dP^T = V dO^T land in TMEM with one
+//                       key per lane, dV += P^T dO and dK += dS^T Q take their left operand straight from TMEM.
+//   dQ   (KV = false):  Q, dO of one 128-row M tile stay (the forward's work items); K, V of the active k-blocks are
+//                       streamed.  S = Q K^T, dP = dO V^T, dQ += dS K.
+// Recomputing S and dP in both launches costs two of seven products but leaves every gradient element with exactly one
+// writer: no fp32 accumulators in memory, no atomics, no conversion pass, and bit-identical results from run to run.
+//
+// P and dS enter the second products as the sum of two 16-bit terms (hi + lo, 16 significant bits for bf16, 22 for fp16),
+// so that no precision is lost against an fp32 product; that doubles three of the seven products, which is what
+// bounds the kernel: per 128x64 tile at d = 128 the tensor pipe is occupied 16 x 47 clocks by the two first products (N = 64
+// operands from shared memory) and 32 x 64 (dK/dV) or 16 x 64 (dQ) by the second ones.  fp16 dS is scaled by a power of two
+// taken from max|dO| max|V| d beforehand, so that neither small nor large (loss-scaled) gradients leave its range.
+//
+// 320 threads, one persistent CTA per SM (TMEM: two tile buffers of 64 S + 64 dP columns, two accumulators of 128):
+//   warps 0-3 / 4-7   elementwise work on the even / odd tiles (thread = TMEM lane), then the epilogue: dV / dK, or the two
+//                     halves of dQ's columns
+//   warp 8            work fetch, mask scan, TMA, and the {-lse, delta} pairs of the streamed rows
+//   warp 9            TMEM allocation and the one thread that issues every tcgen05.mma, in the fixed order
+//                     S(0) dP(0) S(1) dP(1) acc(0) S(2) dP(2) acc(1) ...; S(t+2) overwrites the columns of P(t) right behind
+//                     acc(t) because the instructions of one thread execute in issue order (HBSA_STRICT_TCGEN05 builds wait
+//                     for acc(t) to complete instead).
+// The stationary pair is double buffered (the next item's first products overlap this item's epilogue), the streamed pair
+// has three stages.
+#include <math.h>
+
+#include "sm100_common.cuh"
+
+namespace hbsa {
+
+namespace {
+
+constexpr int kBwdThreads = 320;
+constexpr int kBwdEwWarps = 8;
+constexpr int kBwdProducer = 8;
+constexpr int kBwdMma = 9;
+constexpr int kBwdTile = 64;           // rows of a streamed tile, at most
+constexpr int kBwdStages = 3;
+constexpr uint32_t kBwdBuf = 128u;     // TMEM columns of one S + dP buffer
+constexpr uint32_t kBwdAcc = 256u;     // first accumulator column
+constexpr float kLog2e = 1.4426950408889634f;
+
+// First words of the gradient workspace: work cursors of the two launches, running maxima of |dO| and |V| (float bits).
+struct BwdHeader {
+  unsigned long long cursor[2];
+  unsigned int amax_do, amax_v;
+};
+constexpr size_t kBwdHeaderBytes = 256;
+
+struct BwdParams {
+  Problem p;
+  Workspace ws;
+  BwdHeader* head;
+  const float2* stats;         // [total_q, nhead_q] {-lse * log2 e (-inf: row without keys), delta}
+  void *out0, *out1;           // dv, dk (KV) or dq
+  int total_q, total_k;
+  int gp, gp_shift, n_head_sub;      // q-heads packed into one tile of q rows, tiles of heads per group
+  int tt;                      // tokens per tile of q rows
+  int nt;                      // rows of a streamed tile (multiple of 16)
+  int m_rows, n_msub;          // KV: keys of one stationary tile, tiles per k-block
+  int tiles_per_qblock, items_per_row;  // dQ: as in the forward
+  long long total_items;
+  float scale_log2;
+  long long wait_budget;
+};
+
+struct BwdItem {
+  int n_tiles;                 // < 0: no more work
+  int row0;                    // first stationary row (token) in the packed tensors
+  int end;                     // KV: number of valid keys; dQ: one past the last token of the q-block
+  int head;                    // KV: kv-head; dQ: first q-head
+  int pos0;                    // in-sample position of the first stationary row
+  int k_len, off;
+  int pad;
+};
+
+struct __align__(16) BwdControl {
+  float neg_lse[kBwdStages][kBwdTile];
+  float delta[kBwdStages][kBwdTile];
+  unsigned long long item_full[2], item_done[2], stat_full[2], stat_free[2];
+  unsigned long long strm_full[kBwdStages], strm_free[kBwdStages];
+  unsigned long long s_full[2], dp_full[2], p_ready[2], ds_ready[2];
+  unsigned long long acc_full, acc_free, drain;
+  uint32_t tmem_base;
+  int abort_flag;
+  int info0[kBwdStages], info1[kBwdStages];   // KV: key limit of the tile's first token; dQ: first key, one past the last key
+  BwdItem slot[2];
+};
+
+template <bool BF16> __device__ __forceinline__ void unpack16(uint32_t w, float& a, float& b) {
+  if (BF16) {
+    a = __uint_as_float(w << 16);
+    b = __uint_as_float(w & 0xffff0000u);
+  } else {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    a = f.x;
+    b = f.y;
+  }
+}
+// x0, x1 = hi + lo, two 16-bit terms each
+template <bool BF16> __device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  hi = pack2<BF16>(x0, x1);
+  float h0, h1;
+  unpack16<BF16>(hi, h0, h1);
+  lo = pack2<BF16>(x0 - h0, x1 - h1);
+}
+
+// Power of two that brings |dO V^T| and |delta| below 2^14 (both are bounded by max|dO| max|V| d).
+__device__ __forceinline__ float fp16_grad_factor(const BwdHeader* h, int headdim) {
+  const float bound = __uint_as_float(h->amax_do) * __uint_as_float(h->amax_v) * (float)headdim;
+  if (!(bound > 0.f) || !isfinite(bound)) return 1.f;
+  const int e = 13 - ilogbf(bound);
+  return ldexpf(1.f, e < -60 ? -60 : e > 60 ? 60 : e);
+}
+
+// acc (+)= A[tmem] B over `n` 16-wide k-steps.
+__device__ __forceinline__ void issue_ts(uint32_t acc, uint32_t a_tmem, uint64_t b_desc, int n, uint32_t idesc, bool first) {
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) {
+    if (ks < n) {
+      if (ks == 0 && first) ptx::mma_ts_c<false>(acc, a_tmem, b_desc, idesc);
+      else ptx::mma_ts_c<true>(acc, a_tmem + 8u * ks, b_desc + 128u * ks, idesc);
+    }
+  }
+}
+
+template <int D, bool BF16, bool KV>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_x,
+                 const __grid_constant__ CUtensorMap tm_y, const BwdParams P) {
+  // a, b: stationary pair (K, V or Q, dO); x, y: streamed pair (Q, dO or K, V)
+  using namespace ptx;
+  constexpr int PANELS = D / 64;
+  constexpr uint32_t STAT = 128u * D * 2u, STRM = (uint32_t)kBwdTile * D * 2u;
+  using OutT = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
+  const Problem& p = P.p;
+  OutT* const out0 = static_cast<OutT*>(P.out0);
+  OutT* const out1 = static_cast<OutT*>(P.out1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (P.ws.status[0] != HBSA_STATUS_OK) {       // inconsistent block counts: zero gradients
+    const long long n = KV ? (long long)P.total_k * p.nhead_k * p.headdim : (long long)P.total_q * p.nhead_q * p.headdim;
+    for (long long i = (long long)blockIdx.x * kBwdThreads + tid; i < n; i += (long long)gridDim.x * kBwdThreads) {
+      out0[i] = OutT(0.f);
+      if (KV) out1[i] = OutT(0.f);
+    }
+    return;
+  }
+
+  extern __shared__ __align__(1024) uint8_t smem[];   // 1024-byte aligned tiles for the 128-byte swizzle
+  const uint32_t sStat = smem_u32(smem);              // [2 buffers][a, b]
+  const uint32_t sStrm = sStat + 4 * STAT;            // [stages][x, y]
+  BwdControl* const ctl = reinterpret_cast<BwdControl*>(smem + 4 * STAT + 2 * kBwdStages * STRM);
+  volatile int* const abort_flag = &ctl->abort_flag;
+  const long long budget = P.wait_budget;
+  const uint32_t b_item_full = smem_u32(ctl->item_full), b_item_done = smem_u32(ctl->item_done);
+  const uint32_t b_stat_full = smem_u32(ctl->stat_full), b_stat_free = smem_u32(ctl->stat_free);
+  const uint32_t b_strm_full = smem_u32(ctl->strm_full), b_strm_free = smem_u32(ctl->strm_free);
+  const uint32_t b_s_full = smem_u32(ctl->s_full), b_dp_full = smem_u32(ctl->dp_full);
+  const uint32_t b_p_ready = smem_u32(ctl->p_ready), b_ds_ready = smem_u32(ctl->ds_ready);
+  const uint32_t b_acc_full = smem_u32(&ctl->acc_full), b_acc_free = smem_u32(&ctl->acc_free);
+
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(b_item_full + 8 * i, 1);
+      mbar_init(b_item_done + 8 * i, kBwdEwWarps + 1);
+      mbar_init(b_stat_full + 8 * i, 1);
+      mbar_init(b_stat_free + 8 * i, 1);
+      mbar_init(b_s_full + 8 * i, 1);
+      mbar_init(b_dp_full + 8 * i, 1);
+      mbar_init(b_p_ready + 8 * i, kBwdEwWarps / 2);
+      mbar_init(b_ds_ready + 8 * i, kBwdEwWarps / 2);
+    }
+    for (int i = 0; i < kBwdStages; ++i) {
+      mbar_init(b_strm_full + 8 * i, 1);
+      mbar_init(b_strm_free + 8 * i, 1);
+    }
+    mbar_init(b_acc_full, 1);
+    mbar_init(b_acc_free, kBwdEwWarps);
+    mbar_init(smem_u32(&ctl->drain), 1);
+    // the tiles need a 1024-byte aligned base; without static shared memory the dynamic part has one
+    ctl->abort_flag = (sStat & 1023u) != 0 ? 1 : 0;
+    fence_barrier_init();
+  }
+  if (warp == kBwdMma) {
+    tmem_alloc(smem_u32(&ctl->tmem_base), 512u);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = ctl->tmem_base;
+  const int nt = P.nt;
+  const uint32_t strm_panel = (uint32_t)nt * 128u;
+
+  if (warp == kBwdProducer) {
+    // =============================== work fetch, mask scan, TMA ===============================
+    if (lane == 0) {
+      prefetch_tensormap(&tm_a);
+      prefetch_tensormap(&tm_b);
+      prefetch_tensormap(&tm_x);
+      prefetch_tensormap(&tm_y);
+    }
+    unsigned long long* const cursor = &P.head->cursor[KV ? 1 : 0];
+    int I = 0, Iq = 0, T = 0, stage = 0;
+    uint32_t stage_par = 1u;                       // parity of "stage free" for the current round (first round: free)
+    bool ok = *abort_flag == 0;
+    long long next_idx = 0;
+    if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
+    next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
+
+    auto publish = [&](int n_tiles, int row0, int end, int head, int pos0, int k_len, int off) {
+      if (I >= 2) ok = warp_wait(bar_of(b_item_done, I), par_of(I - 2), abort_flag, budget);
+      if (!ok) return;
+      if (lane == 0) {
+        volatile BwdItem* sl = &ctl->slot[I & 1];
+        sl->n_tiles = n_tiles; sl->row0 = row0; sl->end = end; sl->head = head;
+        sl->pos0 = pos0; sl->k_len = k_len; sl->off = off;
+        __threadfence_block();
+        mbar_arrive(bar_of(b_item_full, I));
+      }
+      ++I;
+    };
+    // stationary pair of the next item with tiles: rows (tokens) from row0, heads from head0
+    auto load_stationary = [&](int row0, int head0) {
+      if (Iq >= 2) ok = warp_wait(bar_of(b_stat_free, Iq), par_of(Iq - 2), abort_flag, budget);
+      if (!ok) return;
+      if (lane == 0) {
+        const uint32_t bar = bar_of(b_stat_full, Iq), dst = sStat + (uint32_t)(Iq & 1) * 2u * STAT;
+        mbar_arrive_expect_tx(bar, 2u * STAT);
+#pragma unroll
+        for (int pn = 0; pn < PANELS; ++pn) {
+          tma_load_3d(dst + pn * 16384u, &tm_a, bar, pn * 64, head0, row0);
+          tma_load_3d(dst + STAT + pn * 16384u, &tm_b, bar, pn * 64, head0, row0);
+        }
+      }
+      ++Iq;
+    };
+    // one streamed tile; KV: `valid` tokens of it are real, their {-lse, delta} pairs go along
+    auto load_tile = [&](int row0, int head0, int valid, int i0, int i1) {
+      float2 st0 = make_float2(-INFINITY, 0.f), st1 = st0;
+      if (KV) {
+        const int c1 = lane + 32, h = P.gp - 1;
+        if ((lane >> P.gp_shift) < valid && lane < nt) st0 = P.stats[(long long)(row0 + (lane >> P.gp_shift)) * p.nhead_q + head0 + (lane & h)];
+        if ((c1 >> P.gp_shift) < valid && c1 < nt) st1 = P.stats[(long long)(row0 + (c1 >> P.gp_shift)) * p.nhead_q + head0 + (c1 & h)];
+      }
+      if (T >= kBwdStages) ok = warp_wait(b_strm_free + 8u * stage, stage_par, abort_flag, budget);
+      if (!ok) return;
+      if (KV) {
+        ctl->neg_lse[stage][lane] = st0.x;
+        ctl->neg_lse[stage][lane + 32] = st1.x;
+        ctl->delta[stage][lane] = st0.y;
+        ctl->delta[stage][lane + 32] = st1.y;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        ctl->info0[stage] = i0;
+        ctl->info1[stage] = i1;
+        __threadfence_block();
+        const uint32_t bar = b_strm_full + 8u * stage, dst = sStrm + (uint32_t)stage * 2u * STRM;
+        mbar_arrive_expect_tx(bar, 2u * (uint32_t)nt * D * 2u);
+#pragma unroll
+        for (int pn = 0; pn < PANELS; ++pn) {
+          tma_load_3d(dst + pn * strm_panel, &tm_x, bar, pn * 64, head0, row0);
+          tma_load_3d(dst + STRM + pn * strm_panel, &tm_y, bar, pn * 64, head0, row0);
+        }
+      }
+      ++T;
+      if (++stage == kBwdStages) {
+        stage = 0;
+        stage_par ^= 1u;
+      }
+    };
+
+    while (ok) {
+      const long long idx = next_idx;
+      if (idx >= P.total_items) {
+        publish(-1, 0, 0, 0, 0, 0, 0);
+        break;
+      }
+      if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
+      next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
+      if (KV) {
+        // item = (kv-head, k-block, sub-tile); under a causal mask the first k-blocks of a sample have the most work
+        const int msub = (int)(idx % P.n_msub);
+        const long long r = idx / P.n_msub;
+        const int kb = (int)(r % p.num_k_block), hk = (int)(r / p.num_k_block);
+        const int b = sample_of_block(P.ws.cnk, p.batch, kb);
+        const int k_begin = p.cu_k[b], k_len = p.cu_k[b + 1] - k_begin, q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
+        const int off = k_len - q_len;
+        const int blk0 = (kb - P.ws.cnk[b]) * p.kbs;
+        const int k0 = blk0 + msub * P.m_rows, k_end = min(blk0 + p.kbs, k_len);
+        if (k0 >= k_end) continue;
+        const int qb0 = P.ws.cnq[b], nqb = P.ws.cnq[b + 1] - qb0;
+        int i_min = 0;
+        if (p.causal) {                             // first q-block whose last row reaches key k0
+          const int need = k0 - off + 1 - p.qbs;    // (i + 1) * qbs - 1 + off >= k0
+          i_min = need > 0 ? min((need + p.qbs - 1) / p.qbs, nqb - 1) : 0;
+        }
+        // tiles of q-block i: token sub-tiles [first, last) x head sub-tiles
+        auto sub_range = [&](int i, int& first, int& last) {
+          const int rows = min(p.qbs, q_len - i * p.qbs);
+          last = (rows + P.tt - 1) / P.tt;
+          first = 0;
+          if (p.causal) {                           // a sub-tile counts when its last token reaches key k0
+            const int t = k0 - off - i * p.qbs;     // first in-block token that does
+            first = t <= 0 ? 0 : t >= rows ? last : t / P.tt;
+          }
+        };
+        auto active = [&](int i) -> bool {
+          if (i >= nqb) return false;
+          if (p.csr_ptr != nullptr) {
+            const long long row = (long long)hk * p.num_q_block + qb0 + i;
+            const int e1 = p.csr_ptr[row + 1];
+            const int e = lower_bound_i32(p.csr_idx, p.csr_ptr[row], e1, kb);
+            return e < e1 && p.csr_idx[e] == kb;
+          }
+          return p.mask[hk * p.mask_s0 + (long long)(qb0 + i) * p.mask_s1 + (long long)kb * p.mask_s2] != 0;
+        };
+        int n_tiles = 0;
+        for (int base = i_min; base < nqb; base += 32) {
+          const int i = base + lane;
+          int first, last;
+          if (active(i)) {
+            sub_range(i, first, last);
+            n_tiles += (last - first) * P.n_head_sub;
+          }
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) n_tiles += __shfl_xor_sync(0xffffffffu, n_tiles, d);
+        publish(n_tiles, k_begin + k0, min(P.m_rows, k_end - k0), hk, k0, k_len, off);
+        if (!ok || n_tiles == 0) continue;
+        load_stationary(k_begin + k0, hk);
+        for (int base = i_min; base < nqb && ok; base += 32) {
+          uint32_t bal = __ballot_sync(0xffffffffu, active(base + lane));
+          while (bal != 0 && ok) {
+            const int i = base + __ffs(bal) - 1;
+            bal &= bal - 1;
+            int first, last;
+            sub_range(i, first, last);
+            const int rows = min(p.qbs, q_len - i * p.qbs);
+            for (int s = first; s < last && ok; ++s)
+              for (int hs = 0; hs < P.n_head_sub && ok; ++hs) {
+                const int t0 = s * P.tt;
+                load_tile(q_begin + i * p.qbs + t0, hk * p.group + hs * P.gp, min(P.tt, rows - t0),
+                          p.causal ? i * p.qbs + t0 + off : 0x7fffffff - 4096, 0);
+              }
+          }
+        }
+      } else {
+        const ItemRecord rec = reinterpret_cast<const ItemRecord*>(P.ws.items)[idx / P.items_per_row];
+        const int rem = (int)(idx % P.items_per_row);
+        const int hsub = rem / P.tiles_per_qblock, qt = rem % P.tiles_per_qblock;
+        const int tok0 = rec.q_begin + qt * P.tt, head0 = rec.hk * p.group + hsub * P.gp;
+        if (tok0 >= rec.q_end) continue;
+        publish(rec.n_tiles, tok0, rec.q_end, head0, rec.q_in0 + qt * P.tt, rec.k_len, rec.off);
+        if (!ok || rec.n_tiles <= 0) continue;
+        load_stationary(tok0, head0);
+        const bool csr = p.csr_ptr != nullptr;
+        const int n_src = csr ? rec.count : rec.n_reach;
+        const uint8_t* mrow = csr ? nullptr : p.mask + rec.hk * p.mask_s0 + rec.qb * p.mask_s1 + (long long)rec.kb0 * p.mask_s2;
+        for (int base = 0; base < n_src && ok; base += 32) {
+          const int jn = base + lane;
+          int val = jn;
+          bool on = jn < n_src;
+          if (csr) val = on ? p.csr_idx[rec.csr_begin + jn] - rec.kb0 : 0;
+          else on = on && mrow[(long long)jn * p.mask_s2] != 0;
+          uint32_t bal = __ballot_sync(0xffffffffu, on);
+          while (bal != 0 && ok) {
+            const int pos = __ffs(bal) - 1;
+            bal &= bal - 1;
+            const int blk0 = __shfl_sync(0xffffffffu, val, pos) * p.kbs;
+            const int k_end = min(blk0 + p.kbs, rec.k_len);
+            for (int k0 = blk0; k0 < k_end && ok; k0 += nt) load_tile(rec.k_begin + k0, rec.hk, nt, k0, k_end);
+          }
+        }
+      }
+    }
+    if (!ok) {                                      // gave up: let the copies already issued land (bounded)
+      for (int back = 1; back <= kBwdStages && T - back >= 0; ++back) {
+        const int c = T - back;
+        mbar_wait_clock(b_strm_full + 8u * (uint32_t)(c % kBwdStages), (uint32_t)(c / kBwdStages) & 1u, budget >> 4);
+      }
+      for (int back = 1; back <= 2 && Iq - back >= 0; ++back)
+        mbar_wait_clock(bar_of(b_stat_full, Iq - back), par_of(Iq - back), budget >> 4);
+    }
+  } else if (warp == kBwdMma) {
+    // =============================== MMA issuer ===============================
+    if (lane == 0 && *abort_flag == 0) {
+      const uint32_t idesc_s = make_idesc(BF16, false, false, 128, nt);
+      const uint32_t idesc_acc = make_idesc(BF16, false, true, 128, D);
+      const int ksteps = nt >> 4;
+      const uint32_t desc_hi = smem_desc_hi(1024u);
+      const uint32_t panel_units = strm_panel >> 4;
+      bool ok = true, fin = false;
+      int sI = 0, sIq = 0, sT = 0, s_left = 0, s_stage = 0;       // S side
+      uint32_t s_par = 0u;
+      bool s_first = false;
+      int aT = 0, aIq = 0, a_stage = 0;                           // accumulator side
+      int fl0 = 0, fl1 = 0;                                       // per tile in flight: bit 0 first, bit 1 last of its item
+
+      // S and dP of the next tile; false when there is none (yet).  While a tile waits for its accumulator products nothing here
+      // blocks: a later item may only be published once the epilogue of an earlier one, which needs those products, is done.
+      auto there = [&](uint32_t bar, uint32_t par) -> bool {
+        if (aT < sT) return mbar_test(bar, par);
+        return ok = mbar_wait_bounded(bar, par, abort_flag, budget);
+      };
+      auto issue_s = [&]() -> bool {
+        while (s_left == 0) {
+          if (fin || !there(bar_of(b_item_full, sI), par_of(sI))) return false;
+          const int n = *(volatile int*)&ctl->slot[sI & 1].n_tiles;
+          mbar_arrive(bar_of(b_item_done, sI));
+          ++sI;
+          fin = n < 0;
+          s_left = n < 0 ? 0 : n;
+          s_first = true;
+        }
+        if (s_first && !there(bar_of(b_stat_full, sIq), par_of(sIq))) return false;
+        if (!there(b_strm_full + 8u * s_stage, s_par)) return false;
+#ifdef HBSA_STRICT_TCGEN05
+        if (sT >= 2) {                              // the products that read P and dS of tile sT - 2 have completed
+          const int c = sT - 2;
+          if (!(ok = mbar_wait_bounded(b_strm_free + 8u * (uint32_t)(c % kBwdStages), (uint32_t)(c / kBwdStages) & 1u, abort_flag, budget))) return false;
+        }
+#endif
+        tc_fence_after();
+        const uint32_t stat = sStat + (uint32_t)(sIq & 1) * 2u * STAT, strm = sStrm + (uint32_t)s_stage * 2u * STRM;
+        const uint32_t tS = tmem + (uint32_t)(sT & 1) * kBwdBuf;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {      // S = a x^T, then dP = b y^T
+          const uint32_t la = smem_desc_lo(stat + half * STAT, 16u), lx = smem_desc_lo(strm + half * STRM, 16u);
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks) {
+            const uint64_t da = smem_desc_join(la + (uint32_t)(ks >> 2) * 1024u + (uint32_t)(ks & 3) * 2u, desc_hi);
+            const uint64_t dx = smem_desc_join(lx + (uint32_t)(ks >> 2) * panel_units + (uint32_t)(ks & 3) * 2u, desc_hi);
+            if (ks == 0) mma_ss_c<false>(tS + half * 64u, da, dx, idesc_s);
+            else mma_ss_c<true>(tS + half * 64u, da, dx, idesc_s);
+          }
+          tc_commit(half == 0 ? bar_of(b_s_full, sT) : bar_of(b_dp_full, sT));
+        }
+        const int fl = (s_first ? 1 : 0) | (s_left == 1 ? 2 : 0);
+        if (sT & 1) fl1 = fl; else fl0 = fl;
+        s_first = false;
+        if (--s_left == 0) {
+          tc_commit(bar_of(b_stat_free, sIq));      // the stationary pair is read by S and dP only
+          ++sIq;
+        }
+        ++sT;
+        if (++s_stage == kBwdStages) {
+          s_stage = 0;
+          s_par ^= 1u;
+        }
+        return true;
+      };
+
+      while (ok) {
+        if (sT < aT + 2 && issue_s()) continue;
+        if (aT == sT) {
+          if (fin) break;
+          continue;                                 // a wait gave up, or items without tiles went by
+        }
+        if (!ok) break;
+        const int fl = (aT & 1) ? fl1 : fl0;
+        const bool first = (fl & 1) != 0;
+        const uint32_t tS = tmem + (uint32_t)(aT & 1) * kBwdBuf, strm = sStrm + (uint32_t)a_stage * 2u * STRM;
+        const uint64_t dx = smem_desc_join(smem_desc_lo(strm, strm_panel), desc_hi);
+        const uint64_t dy = smem_desc_join(smem_desc_lo(strm + STRM, strm_panel), desc_hi);
+        // the first product of an item overwrites the accumulators: the previous epilogue must have read them
+        if (first && aIq >= 1 && !(ok = mbar_wait_bounded(b_acc_free, (uint32_t)(aIq - 1) & 1u, abort_flag, budget))) break;
+        if (KV) {
+          if (!(ok = mbar_wait_bounded(bar_of(b_p_ready, aT), par_of(aT), abort_flag, budget))) break;
+          tc_fence_after();
+          issue_ts(tmem + kBwdAcc, tS, dy, ksteps, idesc_acc, first);
+          issue_ts(tmem + kBwdAcc, tS + 32u, dy, ksteps, idesc_acc, false);
+        }
+        if (!(ok = mbar_wait_bounded(bar_of(b_ds_ready, aT), par_of(aT), abort_flag, budget))) break;
+        tc_fence_after();
+        const uint32_t acc = tmem + kBwdAcc + (KV ? (uint32_t)D : 0u);
+        issue_ts(acc, tS + 64u, dx, ksteps, idesc_acc, first);
+        issue_ts(acc, tS + 96u, dx, ksteps, idesc_acc, false);
+        tc_commit(b_strm_free + 8u * a_stage);
+        if (fl & 2) tc_commit(b_acc_full);
+        if (first) ++aIq;
+        ++aT;
+        if (++a_stage == kBwdStages) a_stage = 0;
+      }
+      tc_commit(smem_u32(&ctl->drain));             // whatever was issued completes before tensor memory is given back
+      mbar_wait_clock(smem_u32(&ctl->drain), 0u, budget);
+    }
+    __syncwarp();
+  } else {
+    // =============================== elementwise + epilogue ===============================
+    const int wg = warp >> 2, row = tid & 127;
+    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
+    const float factor = BF16 ? 1.f : fp16_grad_factor(P.head, p.headdim);
+    const float scale_log2 = P.scale_log2;
+    const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
+    int I = 0, Iq = 0, T = 0, stage = 0;
+    uint32_t stage_par = 0u;
+    bool ok = *abort_flag == 0;
+    while (ok) {
+      ok = warp_wait(bar_of(b_item_full, I), par_of(I), abort_flag, budget);
+      if (!ok) break;
+      volatile BwdItem* sl = &ctl->slot[I & 1];
+      const int n_tiles = sl->n_tiles;
+      if (n_tiles < 0) break;
+      const int row0 = sl->row0, end = sl->end, head = sl->head, pos0 = sl->pos0, k_len = sl->k_len, off = sl->off;
+      // this thread's row of the stationary tile: a key (KV) or a (token, head) pair
+      const int tok = KV ? row0 + row : row0 + (row >> P.gp_shift);
+      const bool valid = KV ? row < end : tok < end;
+      const int hq = KV ? 0 : head + (row & (P.gp - 1));
+      const int key = pos0 + row;
+      float neg_lse = -INFINITY, delta = 0.f;
+      int limit_row = k_len - 1;
+      if (!KV) {
+        if (valid && n_tiles > 0) {
+          const float2 st = P.stats[(long long)tok * p.nhead_q + hq];
+          neg_lse = st.x;
+          delta = st.y;
+        }
+        if (p.causal) limit_row = min(limit_row, pos0 + (row >> P.gp_shift) + off);
+      }
+      for (int t = 0; t < n_tiles && ok; ++t, ++T) {
+        if ((T & 1) == wg) {
+          ok = warp_wait(b_strm_full + 8u * stage, stage_par, abort_flag, budget) && warp_wait(bar_of(b_s_full, T), par_of(T), abort_flag, budget);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t tS = tmem + (uint32_t)(T & 1) * kBwdBuf + lane_off;
+          uint32_t r[64], g[64];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (nt > 16 * j) tmem_ld16(tS + 16 * j, *reinterpret_cast<uint32_t(*)[16]>(&r[16 * j]));
+          // columns this row may not see: below `lo_col` (KV: tokens before the key) or above `hi_col` (dQ: keys past the limit)
+          int lo_col = 0, hi_col = 63;
+          if (KV) {
+            const int lim0 = *(volatile int*)&ctl->info0[stage];
+            if (key > lim0) lo_col = min(key - lim0, 64) << P.gp_shift;
+          } else {
+            const int k0 = *(volatile int*)&ctl->info0[stage], k_end = *(volatile int*)&ctl->info1[stage];
+            hi_col = min(limit_row, k_end - 1) - k0;
+          }
+          const bool edge = KV ? lo_col > 0 : hi_col < nt - 1;
+          tmem_wait_ld();
+          if (__any_sync(0xffffffffu, edge)) {
+#pragma unroll
+            for (int i = 0; i < 64; ++i)
+              if (KV ? i < lo_col : i > hi_col) r[i] = 0xff800000u;     // -inf: its P is an exact zero
+          }
+          const float4* nl4 = reinterpret_cast<const float4*>(ctl->neg_lse[stage]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (nt > 16 * j) {
+              uint32_t hi[8], lo[8];
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                const int c = 16 * j + i;
+                float4 nl = make_float4(neg_lse, neg_lse, neg_lse, neg_lse);
+                if (KV) nl = nl4[c >> 2];
+                float x0, x1, x2, x3;
+                unpack_f32x2(fma_f32x2(pack_b32x2(r[c], r[c + 1]), scale2, pack_f32x2(nl.x, nl.y)), x0, x1);
+                unpack_f32x2(fma_f32x2(pack_b32x2(r[c + 2], r[c + 3]), scale2, pack_f32x2(nl.z, nl.w)), x2, x3);
+                x0 = ex2_approx(x0); x1 = ex2_approx(x1); x2 = ex2_approx(x2); x3 = ex2_approx(x3);
+                if (KV) {
+                  split2<BF16>(x0, x1, hi[i >> 1], lo[i >> 1]);
+                  split2<BF16>(x2, x3, hi[(i >> 1) + 1], lo[(i >> 1) + 1]);
+                }
+                r[c] = __float_as_uint(x0); r[c + 1] = __float_as_uint(x1);
+                r[c + 2] = __float_as_uint(x2); r[c + 3] = __float_as_uint(x3);
+              }
+              if (KV) {
+                tmem_st8(tS + 8 * j, hi);
+                tmem_st8(tS + 32 + 8 * j, lo);
+              }
+            }
+          }
+          if (KV) {
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_of(b_p_ready, T));
+          }
+          ok = warp_wait(bar_of(b_dp_full, T), par_of(T), abort_flag, budget);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (nt > 16 * j) tmem_ld16(tS + 64 + 16 * j, *reinterpret_cast<uint32_t(*)[16]>(&g[16 * j]));
+          tmem_wait_ld();
+          const float4* dl4 = reinterpret_cast<const float4*>(ctl->delta[stage]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (nt > 16 * j) {
+              uint32_t hi[8], lo[8];
+#pragma unroll
+              for (int i = 0; i < 16; i += 4) {
+                const int c = 16 * j + i;
+                float4 dl = make_float4(delta, delta, delta, delta);
+                if (KV) dl = dl4[c >> 2];
+                const float d[4] = {dl.x, dl.y, dl.z, dl.w};
+                float x[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float pr = __uint_as_float(r[c + e]);
+                  x[e] = pr * (__uint_as_float(g[c + e]) - d[e]);
+                  if (!BF16) x[e] *= factor;
+                }
+                split2<BF16>(x[0], x[1], hi[i >> 1], lo[i >> 1]);
+                split2<BF16>(x[2], x[3], hi[(i >> 1) + 1], lo[(i >> 1) + 1]);
+              }
+              tmem_st8(tS + 64 + 8 * j, hi);
+              tmem_st8(tS + 96 + 8 * j, lo);
+            }
+          }
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_of(b_ds_ready, T));
+        }
+        if (++stage == kBwdStages) {
+          stage = 0;
+          stage_par ^= 1u;
+        }
+      }
+      if (!ok) break;
+
+      // ---- epilogue: KV: warpgroup 0 writes dV, 1 writes dK; dQ: each writes half of the columns
+      constexpr int NC = KV ? D : D / 2;
+      const int c_base = KV ? 0 : wg * NC;
+      OutT* const orow = KV ? (wg == 0 ? out0 : out1) + ((long long)tok * p.nhead_k + head) * p.headdim
+                            : out0 + ((long long)tok * p.nhead_q + hq) * p.headdim;
+      const float mul = KV && wg == 0 ? 1.f : p.scale / factor;
+      if (n_tiles > 0) {
+        ok = warp_wait(b_acc_full, (uint32_t)Iq & 1u, abort_flag, budget);
+        if (!ok) break;
+        tc_fence_after();
+      }
+      const uint32_t tA = tmem + kBwdAcc + (uint32_t)(wg * NC) + lane_off;
+#pragma unroll
+      for (int cb = 0; cb < NC; cb += 32) {
+        uint32_t a[32];
+        if (n_tiles > 0) {
+          tmem_ld32(tA + cb, a);
+          tmem_wait_ld();
+          if (cb + 32 >= NC) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(b_acc_free);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) a[i] = 0u;
+        }
+        if (valid) {
+#pragma unroll
+          for (int c = 0; c < 32; c += 8) {
+            if (c_base + cb + c < p.headdim) {
+              uint32_t w[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) w[e] = pack2<BF16>(__uint_as_float(a[c + 2 * e]) * mul, __uint_as_float(a[c + 2 * e + 1]) * mul);
+              *reinterpret_cast<uint4*>(orow + c_base + cb + c) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+          }
+        }
+      }
+      if (n_tiles > 0) ++Iq;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar_of(b_item_done, I));
+      ++I;
+    }
+  }
+
+  // ---- teardown: every thread gets here (all waits are bounded)
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kBwdMma) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512u);
+  }
+  if (tid == 0 && ctl->abort_flag) {
+    atomicExch(&P.ws.status[0], HBSA_STATUS_WAIT_LIMIT);
+    P.ws.status[3] = (int)blockIdx.x;
+  }
+}
+
+// {-lse * log2 e, delta = rowsum(dO * O)} of every (token, q-head) row; with fp16 also max|dO| and max|V|.  16 lanes per row, 16
+// bytes per lane; bound by the read of O and dO.  Rows of q / k outside every sample get zero gradients here.
+template <bool BF16>
+__global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams P, const uint16_t* __restrict__ o, long long o0, long long o1,
+                                                       const uint16_t* __restrict__ d_o, long long g0, long long g1,
+                                                       const uint16_t* __restrict__ v, long long v0, long long v1,
+                                                       const float* __restrict__ lse, float2* __restrict__ stats, uint16_t* dq, uint16_t* dk, uint16_t* dv) {
+  const Problem& p = P.p;
+  const int chunk = threadIdx.x & 15, n_chunk = p.headdim >> 3;
+  const long long first = (long long)blockIdx.x * 16 + (threadIdx.x >> 4), step = (long long)gridDim.x * 16;
+  const long long rows = (long long)P.total_q * p.nhead_q;
+  float am = 0.f, vm = 0.f;
+  const int q_lo = p.cu_q[0], q_hi = p.cu_q[p.batch], k_lo = p.cu_k[0], k_hi = p.cu_k[p.batch];
+  for (long long base = (long long)blockIdx.x * 16; base < rows; base += step) {      // uniform per block: the shuffles need whole warps
+    const long long row = base + (threadIdx.x >> 4);
+    float acc = 0.f;
+    const long long tok = row / p.nhead_q, h = row % p.nhead_q;
+    if (row < rows && chunk < n_chunk) {
+      const uint4 a = *reinterpret_cast<const uint4*>(o + tok * o0 + h * o1 + chunk * 8);
+      const uint4 b = *reinterpret_cast<const uint4*>(d_o + tok * g0 + h * g1 + chunk * 8);
+      const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float x0, x1, y0, y1;
+        unpack16<BF16>(wa[i], x0, x1);
+        unpack16<BF16>(wb[i], y0, y1);
+        acc = fmaf(x0, y0, fmaf(x1, y1, acc));
+        if (!BF16) am = fmaxf(am, fmaxf(fabsf(y0), fabsf(y1)));
+      }
+    }
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (row < rows) {
+      if (chunk == 0) {
+        const float l = lse[row];
+        stats[row] = l > -INFINITY ? make_float2(-l * kLog2e, acc) : make_float2(-INFINITY, 0.f);
+      }
+      if ((tok < q_lo || tok >= q_hi) && chunk < n_chunk) *reinterpret_cast<uint4*>(dq + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
+    }
+  }
+  const long long k_rows = (long long)P.total_k * p.nhead_k;
+  for (long long row = first; row < k_rows; row += step) {
+    const long long tok = row / p.nhead_k, h = row % p.nhead_k;
+    if (chunk < n_chunk && (tok < k_lo || tok >= k_hi)) {
+      *reinterpret_cast<uint4*>(dk + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
+      *reinterpret_cast<uint4*>(dv + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
+    }
+    if (!BF16 && chunk < n_chunk) {
+      const uint4 a = *reinterpret_cast<const uint4*>(v + tok * v0 + h * v1 + chunk * 8);
+      const uint32_t wa[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float x0, x1;
+        unpack16<BF16>(wa[i], x0, x1);
+        vm = fmaxf(vm, fmaxf(fabsf(x0), fabsf(x1)));
+      }
+    }
+  }
+  if (!BF16) {                                       // maxima of non-negative floats order like their bits
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, s));
+      vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, s));
+    }
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(&P.head->amax_do, __float_as_uint(am));
+      atomicMax(&P.head->amax_v, __float_as_uint(vm));
+    }
+  }
+}
+
+// q-heads packed into a tile of at most `rows` rows: the largest power of two that divides the group
+int pack_heads(int group, int rows) {
+  int gp = 1;
+  while (gp < rows && group % (gp * 2) == 0) gp *= 2;
+  return gp;
+}
+int log2_of(int x) {
+  int s = 0;
+  while ((1 << s) < x) ++s;
+  return s;
+}
+// rows of a streamed tile: `rows` split evenly into the fewest tiles of at most 64, rounded up to 16
+int even_tile(int rows) {
+  const int n = (rows + kBwdTile - 1) / kBwdTile;
+  return ((rows + n - 1) / n + 15) / 16 * 16;
+}
+
+template <int D, bool BF16, bool KV>
+cudaError_t launch_one(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& x, const CUtensorMap& y, const BwdParams& P, cudaStream_t stream) {
+  constexpr size_t smem = 4u * 128u * D * 2u + 2u * kBwdStages * kBwdTile * D * 2u + sizeof(BwdControl);
+  static_assert(smem <= 227u * 1024u, "shared memory of one CTA");
+  cudaError_t e = cudaFuncSetAttribute(bwd_sm100_kernel<D, BF16, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const long long resident = sm100_sm_count();
+  const unsigned grid = (unsigned)(P.total_items < resident ? P.total_items : resident);
+  bwd_sm100_kernel<D, BF16, KV><<<grid, kBwdThreads, smem, stream>>>(a, b, x, y, P);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+size_t backward_sm100_workspace_bytes(long long total_q, int nhead_q) {
+  return kBwdHeaderBytes + (size_t)(total_q * nhead_q) * sizeof(float2);
+}
+
+const char* backward_sm100_ineligible_reason(const hbsa_backward_args& b, float scale) {
+  const char* why = sm100_ineligible_reason(b.fwd, scale);
+  if (why) return why;
+  if (b.fwd.headdim > 128) return "headdim is above 128";
+  if (b.do_stride[2] != 1) return "headdim stride of d_o is not 1";
+  for (int i = 0; i < 2; ++i)
+    if (b.do_stride[i] <= 0 || (b.do_stride[i] * 2) % 16 != 0) return "a token/head stride of d_o is not a positive multiple of 16 bytes";
+  if ((uintptr_t)b.d_o % 16 != 0 || (uintptr_t)b.dq % 16 != 0 || (uintptr_t)b.dk % 16 != 0 || (uintptr_t)b.dv % 16 != 0)
+    return "a gradient's base address is not 16-byte aligned";
+  return nullptr;
+}
+
+int backward_sm100_kv_tile_rows(int kbs) { return even_tile(kbs); }
+
+int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_backward_args& b, cudaStream_t stream, const char** err_text) {
+  const hbsa_forward_args& a = b.fwd;
+  EncodeTiledFn fn = sm100_encode_fn();
+  if (!fn) { *err_text = "cuTensorMapEncodeTiled is not available from the CUDA driver"; return HBSA_ERR_DRIVER; }
+  const bool bf16 = a.dtype == HBSA_DTYPE_BF16;
+  BwdParams P = {};
+  P.p = p;
+  P.ws = ws;
+  P.head = static_cast<BwdHeader*>(b.grad_workspace);
+  float2* stats = reinterpret_cast<float2*>(static_cast<char*>(b.grad_workspace) + kBwdHeaderBytes);
+  P.stats = stats;
+  P.total_q = a.total_q;
+  P.total_k = a.total_k;
+  P.scale_log2 = p.scale * kLog2e;
+  P.wait_budget = sm100_wait_budget();
+  cudaError_t e = cudaMemsetAsync(P.head, 0, sizeof(BwdHeader), stream);
+  if (e != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
+  {
+    const long long rows = (long long)a.total_q * a.nhead_q;
+    const long long blocks = (rows + 15) / 16, most = 16ll * sm100_sm_count();
+    const unsigned grid = (unsigned)(blocks < most ? blocks : most);
+    const uint16_t *o = static_cast<const uint16_t*>(a.o), *d_o = static_cast<const uint16_t*>(b.d_o), *v = static_cast<const uint16_t*>(a.v);
+    uint16_t *dq = static_cast<uint16_t*>(b.dq), *dk = static_cast<uint16_t*>(b.dk), *dv = static_cast<uint16_t*>(b.dv);
+    if (bf16) bwd_prep_kernel<true><<<grid, 256, 0, stream>>>(P, o, a.o_stride[0], a.o_stride[1], d_o, b.do_stride[0], b.do_stride[1], v, a.v_stride[0], a.v_stride[1], a.lse, stats, dq, dk, dv);
+    else bwd_prep_kernel<false><<<grid, 256, 0, stream>>>(P, o, a.o_stride[0], a.o_stride[1], d_o, b.do_stride[0], b.do_stride[1], v, a.v_stride[0], a.v_stride[1], a.lse, stats, dq, dk, dv);
+    if ((e = cudaGetLastError()) != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
+  }
+  for (int kv = 0; kv < 2; ++kv) {
+    if (kv) {
+      P.gp = pack_heads(p.group, kBwdTile);
+      P.tt = even_tile(p.qbs * P.gp) / P.gp;        // tokens x heads of a q-block, split evenly
+      P.nt = P.tt * P.gp;
+      P.n_msub = (p.kbs + 127) / 128;
+      P.m_rows = ((p.kbs + P.n_msub - 1) / P.n_msub + 15) / 16 * 16;
+      P.total_items = (long long)p.nhead_k * p.num_k_block * P.n_msub;
+      P.out0 = b.dv;
+      P.out1 = b.dk;
+    } else {
+      P.gp = pack_heads(p.group, 128);
+      P.tt = 128 / P.gp;
+      P.nt = p.kv_tile;
+      P.tiles_per_qblock = (p.qbs + P.tt - 1) / P.tt;
+      P.items_per_row = p.group / P.gp * P.tiles_per_qblock;
+      P.total_items = (long long)p.nhead_k * p.num_q_block * P.items_per_row;
+      P.out0 = b.dq;
+      P.out1 = nullptr;
+    }
+    P.gp_shift = log2_of(P.gp);
+    P.n_head_sub = p.group / P.gp;
+    CUtensorMap q, g, k, v;
+    const int qh = P.gp, qt = P.tt, kt = kv ? 128 : P.nt;
+    if (!sm100_encode_map(fn, &q, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], qh, qt) ||
+        !sm100_encode_map(fn, &g, bf16, b.d_o, p.headdim, p.nhead_q, a.total_q, b.do_stride[0], b.do_stride[1], qh, qt) ||
+        !sm100_encode_map(fn, &k, bf16, a.k, p.headdim, p.nhead_k, a.total_k, a.k_stride[0], a.k_stride[1], 1, kt) ||
+        !sm100_encode_map(fn, &v, bf16, a.v, p.headdim, p.nhead_k, a.total_k, a.v_stride[0], a.v_stride[1], 1, kt)) {
+      *err_text = "cuTensorMapEncodeTiled rejected a q/k/v/d_o layout";
+      return HBSA_ERR_UNSUPPORTED;
+    }
+#define HBSA_LAUNCH_BWD(D_, BF_) (kv ? launch_one<D_, BF_, true>(k, v, q, g, P, stream) : launch_one<D_, BF_, false>(q, g, k, v, P, stream))
+    if (p.headdim <= 64) e = bf16 ? HBSA_LAUNCH_BWD(64, true) : HBSA_LAUNCH_BWD(64, false);
+    else e = bf16 ? HBSA_LAUNCH_BWD(128, true) : HBSA_LAUNCH_BWD(128, false);
+#undef HBSA_LAUNCH_BWD
+    if (e != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
+  }
+  return 0;
+}
+
+}  // namespace hbsa

@@ -124,6 +124,16 @@ __device__ __forceinline__ int lower_bound_i32(const int32_t* __restrict__ a, in
   return lo;
 }
 
+// Largest b with cnb[b] <= blk  (cnb is non-decreasing, cnb[0] = 0, blk < cnb[batch]).
+__device__ __forceinline__ int sample_of_block(const int32_t* __restrict__ cnb, int batch, int blk) {
+  int lo = 0, hi = batch;          // invariant: cnb[lo] <= blk < cnb[hi]
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (cnb[mid] <= blk) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
 // printf-style setter of the text hbsa_last_error() returns on the calling thread.
 void set_last_error(const char* fmt, ...);
 
@@ -144,6 +154,12 @@ cudaError_t launch_forward_generic(const Problem& p, const Workspace& ws, const 
                                    cudaStream_t stream);
 size_t backward_workspace_bytes(long long total_q, long long total_k, int nhead_q, int nhead_k, int headdim);
 cudaError_t launch_backward_generic(const Problem& p, const Workspace& ws, const hbsa_backward_args& b, cudaStream_t stream);
+// Backward on the tensor cores (bf16 / fp16, head dimensions up to 128); same conventions as the forward's functions below.
+size_t backward_sm100_workspace_bytes(long long total_q, int nhead_q);
+const char* backward_sm100_ineligible_reason(const hbsa_backward_args& b, float scale);
+// Rows of one streamed K/V tile; the schedule's tile counts must be made for it (Problem::kv_tile).
+int backward_sm100_kv_tile_rows(int kbs);
+int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_backward_args& b, cudaStream_t stream, const char** err_text);
 // Returns nullptr when eligible, else a static string saying why not.
 const char* sm100_ineligible_reason(const hbsa_forward_args& a, float scale);
 // err_text receives a message when a negative HBSA_ERR_* is returned.

@@ -49,15 +49,12 @@
 // reset): the issuing thread reads it with an ordinary load in its polling loop.
 //   q_full [Iq]: Q tile landed                     o_free [Iq]: epilogue has read O out of TMEM
 //   item_full [I]: item slot written               item_done [I]: all consumers left item I
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <math.h>
 #include <stdlib.h>
 #include <mutex>
 #include <type_traits>
 
-#include "hbsa_common.cuh"
-#include "sm100_ptx.cuh"
+#include "sm100_common.cuh"
 
 namespace hbsa {
 
@@ -129,12 +126,6 @@ struct __align__(16) Control {
   ItemSlot slot[2];
 };
 
-template <bool BF16> __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  uint32_t r;
-  if (BF16) asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-  else asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-  return r;
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
@@ -173,16 +164,6 @@ __device__ __forceinline__ void exp16(const uint32_t* r, uint32_t (&pk)[8], floa
   ptx::unpack_f32x2(sa, sum[0], sum[2]);
   ptx::unpack_f32x2(sb, sum[1], sum[3]);
 }
-
-// One lane polls the mbarrier, the rest of the warp sleeps at the shuffle instead of spinning.
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, long long budget) {
-  int ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = ptx::mbar_wait_bounded(bar, parity, abort_flag, budget) ? 1 : 0;
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
-// Barrier entry and parity for the c-th use of a two-entry barrier array.
-__device__ __forceinline__ uint32_t bar_of(uint32_t base, int c) { return base + 8u * (uint32_t)(c & 1); }
-__device__ __forceinline__ uint32_t par_of(int c) { return (uint32_t)(c >> 1) & 1u; }
 
 // The issue sequences of the MMA thread.  Every descriptor and TMEM address is precomputed into
 // registers once per CTA, so a product is nothing but back-to-back tcgen05.mma instructions.
@@ -815,11 +796,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 }
 
 // ------------------------------------------------------------------------------------------ host
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+long long* g_trace = nullptr;
+long long g_wait_budget = 4000000000ll;   // clock64 ticks a wait inside the kernel may take (about two seconds)
+int g_debug_stall = 0;
 
-EncodeTiledFn get_encode_fn() {
+}  // namespace
+
+EncodeTiledFn sm100_encode_fn() {
   static EncodeTiledFn fn = nullptr;
   static std::once_flag once;
   std::call_once(once, [] {
@@ -833,7 +816,7 @@ EncodeTiledFn get_encode_fn() {
 }
 
 // 3-D map over a [tokens, heads, headdim] tensor: dims (headdim, heads, tokens), box (64, box_heads, box_tokens).
-bool encode_map(EncodeTiledFn fn, CUtensorMap* map, bool bf16, const void* base, int headdim, int heads, int tokens,
+bool sm100_encode_map(EncodeTiledFn fn, CUtensorMap* map, bool bf16, const void* base, int headdim, int heads, int tokens,
                 long long s_tok, long long s_head, int box_heads, int box_tokens) {
   cuuint64_t dims[3] = {(cuuint64_t)headdim, (cuuint64_t)heads, (cuuint64_t)tokens};
   cuuint64_t strides[2] = {(cuuint64_t)s_head * 2ull, (cuuint64_t)s_tok * 2ull};
@@ -845,11 +828,7 @@ bool encode_map(EncodeTiledFn fn, CUtensorMap* map, bool bf16, const void* base,
   return r == CUDA_SUCCESS;
 }
 
-long long* g_trace = nullptr;
-long long g_wait_budget = 4000000000ll;   // clock64 ticks a wait inside the kernel may take (about two seconds)
-int g_debug_stall = 0;
-
-int sm_count() {
+int sm100_sm_count() {
   static int cached[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
@@ -861,8 +840,7 @@ int sm_count() {
   return cached[dev];
 }
 
-}  // namespace
-
+long long sm100_wait_budget() { return g_wait_budget; }
 void sm100_set_wait_budget(long long clocks, int stall_producer) {
   g_wait_budget = clocks > 0 ? clocks : 4000000000ll;
   g_debug_stall = stall_producer ? 1 : 0;
@@ -895,7 +873,7 @@ const char* sm100_ineligible_reason(const hbsa_forward_args& a, float scale) {
 
 int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forward_args& a, cudaStream_t stream,
                          const char** err_text) {
-  EncodeTiledFn fn = get_encode_fn();
+  EncodeTiledFn fn = sm100_encode_fn();
   if (!fn) { *err_text = "cuTensorMapEncodeTiled is not available from the CUDA driver"; return HBSA_ERR_DRIVER; }
   const bool bf16 = a.dtype == HBSA_DTYPE_BF16;
 
@@ -928,13 +906,13 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   if (P.total_items <= 0) { *err_text = "no work items"; return HBSA_ERR_SHAPE; }
   // two persistent CTAs per SM; one above 128 head dimensions (O alone takes 256 of the SM's 512 TMEM columns, the
   // tiles 192 KB of its shared memory)
-  const long long resident = (p.headdim > 128 ? 1ll : 2ll) * sm_count();
+  const long long resident = (p.headdim > 128 ? 1ll : 2ll) * sm100_sm_count();
   const unsigned grid = (unsigned)(P.total_items < resident ? P.total_items : resident);
 
   CUtensorMap tq, tk, tv;
-  if (!encode_map(fn, &tq, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], gp, P.tt) ||
-      !encode_map(fn, &tk, bf16, a.k, p.headdim, p.nhead_k, a.total_k, a.k_stride[0], a.k_stride[1], 1, P.nt) ||
-      !encode_map(fn, &tv, bf16, a.v, p.headdim, p.nhead_k, a.total_k, a.v_stride[0], a.v_stride[1], 1, P.nt)) {
+  if (!sm100_encode_map(fn, &tq, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], gp, P.tt) ||
+      !sm100_encode_map(fn, &tk, bf16, a.k, p.headdim, p.nhead_k, a.total_k, a.k_stride[0], a.k_stride[1], 1, P.nt) ||
+      !sm100_encode_map(fn, &tv, bf16, a.v, p.headdim, p.nhead_k, a.total_k, a.v_stride[0], a.v_stride[1], 1, P.nt)) {
     *err_text = "cuTensorMapEncodeTiled rejected a q/k/v layout";
     return HBSA_ERR_UNSUPPORTED;
   }

@@ -89,16 +89,6 @@ __global__ void __launch_bounds__(1024) calc_num_blocks_kernel(const int32_t* __
   scan_num_blocks(cu, batch, bs, cu_num_block);
 }
 
-// Largest b with cnb[b] <= blk  (cnb is non-decreasing, cnb[0] = 0, blk < cnb[batch]).
-__device__ __forceinline__ int sample_of_block(const int32_t* __restrict__ cnb, int batch, int blk) {
-  int lo = 0, hi = batch;          // invariant: cnb[lo] <= blk < cnb[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (cnb[mid] <= blk) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
 __global__ void fill_blocks_kernel(const int32_t* __restrict__ cu, int batch, int bs, int capacity,
                                    const int32_t* __restrict__ cnb, int32_t* __restrict__ cu_block,
                                    int32_t* __restrict__ block_to_batch) {
@@ -207,7 +197,7 @@ __global__ void __launch_bounds__(256) sched_count_kernel(Problem p, Workspace w
     ws.counts[row] = cnt;
     int n_tiles = cnt;
     if (p.kv_tile > 0 && p.kv_tile < p.kbs) {
-      const int n_sub = p.kbs / p.kv_tile;
+      const int n_sub = (p.kbs + p.kv_tile - 1) / p.kv_tile;
       n_tiles = cnt * n_sub;
       if (last_active) {
         const int len_last = g.k_len - j_last * p.kbs;

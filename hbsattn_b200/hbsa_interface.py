@@ -201,6 +201,8 @@ def attention_backward(q, k, v, out, lse, d_out, cu_q_seqlens, cu_k_seqlens, blo
     cu_q32, cu_k32 = _prepare(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask)
     if d_out.dtype != q.dtype:
         d_out = d_out.to(q.dtype)
+    if d_out.stride(2) != 1 or any(n <= 0 or n % 8 for n in d_out.stride()[:2]):
+        d_out = d_out.contiguous()                   # an expanded or transposed gradient: the tensor-core kernel loads 16-byte rows
     nqb = block_mask.shape[1] if num_q_block is None else num_q_block
     nkb = block_mask.shape[2] if num_k_block is None else num_k_block
     lib = _lib.load()

@@ -178,8 +178,10 @@ int hbsa_block_decisions(const hbsa_forward_args* args, uint8_t* decisions, int3
  *            (required: run the forward with lse set), mask, sizes, workspace (the schedule is rebuilt in it)
  *   d_o      gradient of the output, same dtype as q, [total_q, nhead_q, headdim] with element strides do_stride
  *   dq, dk, dv   results in the dtype of q, contiguous [total_q, nhead_q, headdim] / [total_k, nhead_k, headdim]
- *   grad_workspace   >= hbsa_backward_workspace_bytes(...) bytes of device memory (fp32 accumulators), 256-byte aligned
- * CUDA-core kernels for every dtype and headdim <= 256; rows that saw no key get zero gradients.
+ *   grad_workspace   >= hbsa_backward_workspace_bytes(...) bytes of device memory, 256-byte aligned
+ * The tcgen05 backward runs bf16/fp16 problems the forward's tcgen05 kernel takes, up to headdim 128 (d_o, dq, dk, dv with
+ * 16-byte aligned rows); CUDA-core kernels with fp32 accumulators in grad_workspace run the rest (headdim <= 256).  fwd.impl
+ * forces one of the two as in the forward.  Rows that saw no key get zero gradients.
  */
 typedef struct hbsa_backward_args {
   size_t struct_bytes;            /* sizeof(hbsa_backward_args) of the caller */
