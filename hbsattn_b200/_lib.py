@@ -22,8 +22,10 @@ EXPORTED_SYMBOLS = (
     "hbsa_version",
     "hbsa_last_error",
     "hbsa_calculate_blocks",
+    "hbsa_calculate_blocks_counted",
     "hbsa_workspace_bytes",
     "hbsa_forward",
+    "hbsa_forward_status",
     "hbsa_build_schedule",
     "hbsa_attention",
     "hbsa_block_decisions",
@@ -124,6 +126,10 @@ def load() -> ctypes.CDLL:
         lib.hbsa_workspace_bytes.argtypes = [i32, i32, i32, i32]
         lib.hbsa_forward.restype = i32
         lib.hbsa_forward.argtypes = [ctypes.POINTER(ForwardArgs), vp]
+        lib.hbsa_forward_status.restype = i32
+        lib.hbsa_forward_status.argtypes = [ctypes.POINTER(ForwardArgs), vp, vp]
+        lib.hbsa_calculate_blocks_counted.restype = i32
+        lib.hbsa_calculate_blocks_counted.argtypes = [vp, i32, i32, i32, vp, vp, vp, vp, vp]
         for name in ("hbsa_build_schedule", "hbsa_attention"):
             getattr(lib, name).restype = i32
             getattr(lib, name).argtypes = [ctypes.POINTER(ForwardArgs), vp]
@@ -151,6 +157,22 @@ def load() -> ctypes.CDLL:
             raise ImportError("libhbsattn_b200.so was built from a different ABI version")
         _lib = lib
         return lib
+
+
+# Order of struct Library in csrc/hbsa_host.cpp.
+_HOST_FUNCTIONS = ("hbsa_forward", "hbsa_forward_status", "hbsa_attention", "hbsa_backward", "hbsa_calculate_blocks_counted",
+                   "hbsa_calculate_blocks", "hbsa_workspace_bytes", "hbsa_backward_workspace_bytes", "hbsa_last_error")
+
+
+def load_host(state: dict):
+    """The host extension, bound to the library ``load`` has loaded; raises if it has not been built."""
+    lib = load()
+    try:
+        from . import _host
+    except ImportError as e:
+        raise ImportError(f"hbsattn_b200/_host.so cannot be loaded ({e}): build it with `python hbsattn_b200/build.py`") from e
+    _host.setup(state, tuple(ctypes.cast(getattr(lib, name), ctypes.c_void_p).value for name in _HOST_FUNCTIONS))
+    return _host
 
 
 def last_error() -> str:

@@ -80,6 +80,67 @@ int select_impl(const hbsa_forward_args* a, const hbsa::Problem& p) {
   return why ? HBSA_IMPL_GENERIC : HBSA_IMPL_SM100;
 }
 
+// Mapped host memory a kernel reports to, so that a call that has to wait for a few words neither copies them nor waits for the
+// stream's own completion machinery.  One block per host thread, reused by its calls one after the other and freed with the
+// thread; the tag tells a report from an older one.
+struct HostWords {
+  volatile int32_t* words = nullptr;
+  int tag = 0;
+  ~HostWords() {
+    if (words) cudaFreeHost(const_cast<int32_t*>(words));
+  }
+  int next() { return tag = tag == 0x7fffffff ? 1 : tag + 1; }
+  bool there() const { return __atomic_load_n(const_cast<int32_t*>(words), __ATOMIC_ACQUIRE) == tag; }
+  // Until the report with the last tag is there; asks the stream now and then, so that a failed launch ends the wait.
+  int wait(cudaStream_t stream, const char* where) const {
+    for (unsigned long long i = 1;; ++i) {
+      if (there()) return 0;
+      if ((i & 4095u) == 0) {
+        const cudaError_t e = cudaStreamQuery(stream);
+        if (e == cudaSuccess) return there() ? 0 : fail(HBSA_ERR_DRIVER, "the stream finished without the kernel's report");
+        if (e != cudaErrorNotReady) return fail_cuda(e, where);
+      }
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+    }
+  }
+};
+
+HostWords* host_words() {
+  static thread_local HostWords w;
+  if (!w.words) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, 64, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return nullptr;
+    memset(p, 0, 64);
+    w.words = static_cast<int32_t*>(p);
+  }
+  return &w;
+}
+
+// The forward with or without building its schedule first; everything is rejected before the first launch.  With `report` the
+// status words go to the host when the attention kernel is through (the caller waits for them).
+int forward(const hbsa_forward_args* args, bool schedule, HostWords* report, cudaStream_t stream) {
+  hbsa::Problem p;
+  int rc = make_problem(args, true, &p);
+  if (rc != 0) return rc;
+  const int impl = select_impl(args, p);
+  if (impl < 0) return impl;
+  hbsa::Workspace ws = hbsa::make_workspace(args->workspace, p.nhead_k, p.num_q_block, p.num_k_block, p.batch);
+  cudaError_t e = cudaSuccess;
+  if (schedule && (e = hbsa::launch_schedule(p, ws, nullptr, stream)) != cudaSuccess) return fail_cuda(e, "hbsa_forward (schedule)");
+  int32_t* const words = report ? const_cast<int32_t*>(report->words) : nullptr;
+  const int tag = report ? report->next() : 0;
+  if (impl == HBSA_IMPL_SM100) {
+    const char* text = "";
+    rc = hbsa::launch_forward_sm100(p, ws, *args, stream, words, tag, &text);
+    return rc != 0 ? fail(rc, text) : 0;
+  }
+  e = hbsa::launch_forward_generic(p, ws, *args, stream);
+  if (e == cudaSuccess && words) e = hbsa::launch_notify(ws, words, tag, stream);
+  return e == cudaSuccess ? 0 : fail_cuda(e, "hbsa_forward (generic kernel)");
+}
+
 }  // namespace
 
 namespace hbsa {
@@ -130,32 +191,43 @@ int hbsa_build_schedule(const hbsa_forward_args* args, void* stream_) {
   return e == cudaSuccess ? 0 : fail_cuda(e, "hbsa_build_schedule");
 }
 
-int hbsa_attention(const hbsa_forward_args* args, void* stream_) {
-  hbsa::Problem p;
-  int rc = make_problem(args, true, &p);
+int hbsa_attention(const hbsa_forward_args* args, void* stream) { return forward(args, false, nullptr, static_cast<cudaStream_t>(stream)); }
+
+int hbsa_forward(const hbsa_forward_args* args, void* stream) { return forward(args, true, nullptr, static_cast<cudaStream_t>(stream)); }
+
+int hbsa_forward_status(const hbsa_forward_args* args, int32_t* status_out, void* stream) {
+  if (!status_out) return fail(HBSA_ERR_NULL, "status_out must not be NULL");
+  HostWords* w = host_words();
+  if (!w) return fail((int)cudaErrorMemoryAllocation, "hbsa_forward_status: no mapped host memory for the status words");
+  int rc = forward(args, true, w, static_cast<cudaStream_t>(stream));
   if (rc != 0) return rc;
-  const int impl = select_impl(args, p);
-  if (impl < 0) return impl;
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  hbsa::Workspace ws = hbsa::make_workspace(args->workspace, p.nhead_k, p.num_q_block, p.num_k_block, p.batch);
-  if (impl == HBSA_IMPL_SM100) {
-    const char* text = "";
-    rc = hbsa::launch_forward_sm100(p, ws, *args, stream, &text);
-    return rc != 0 ? fail(rc, text) : 0;
-  }
-  cudaError_t e = hbsa::launch_forward_generic(p, ws, *args, stream);
-  return e == cudaSuccess ? 0 : fail_cuda(e, "hbsa_attention (generic kernel)");
+  rc = w->wait(static_cast<cudaStream_t>(stream), "hbsa_forward_status");
+  if (rc != 0) return rc;
+  for (int i = 0; i < hbsa::kStatusWords; ++i) status_out[i] = i < hbsa::kNotifyWords - 1 ? w->words[1 + i] : 0;
+  return 0;
 }
 
-int hbsa_forward(const hbsa_forward_args* args, void* stream) {
-  hbsa::Problem p;
-  int rc = make_problem(args, true, &p);          // reject everything before the first launch
-  if (rc != 0) return rc;
-  rc = select_impl(args, p);
-  if (rc < 0) return rc;
-  rc = hbsa_build_schedule(args, stream);
-  if (rc != 0) return rc;
-  return hbsa_attention(args, stream);
+int hbsa_calculate_blocks_counted(const int32_t* cu_seqlen, int batch, int block_size, int capacity, int32_t* cu_block,
+                                  int32_t* block_to_batch, int32_t* cu_num_block, int32_t* num_block, void* stream_) {
+  if (!cu_seqlen || !cu_num_block || !cu_block || !block_to_batch || !num_block) return fail(HBSA_ERR_NULL, "no pointer may be NULL");
+  if (batch <= 0 || capacity < 0) return fail(HBSA_ERR_SHAPE, "batch must be positive and capacity non-negative");
+  if (block_size <= 0) return fail(HBSA_ERR_BLOCK_SIZE, "block_size must be positive");
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (!hbsa::calculate_blocks_fits_one_launch(batch)) {
+    cudaError_t e = hbsa::launch_calculate_blocks(cu_seqlen, batch, block_size, capacity, cu_block, block_to_batch, cu_num_block, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(num_block, cu_num_block + batch, sizeof(int32_t), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    return e == cudaSuccess ? 0 : fail_cuda(e, "hbsa_calculate_blocks_counted");
+  }
+  HostWords* w = host_words();
+  if (!w) return fail((int)cudaErrorMemoryAllocation, "hbsa_calculate_blocks_counted: no mapped host memory");
+  const int tag = w->next();
+  cudaError_t e = hbsa::launch_count_and_fill(cu_seqlen, batch, block_size, capacity, cu_block, block_to_batch, cu_num_block,
+                                              const_cast<int32_t*>(w->words), tag, stream);
+  if (e != cudaSuccess) return fail_cuda(e, "hbsa_calculate_blocks_counted");
+  const int rc = w->wait(stream, "hbsa_calculate_blocks_counted");
+  if (rc == 0) *num_block = w->words[1];
+  return rc;
 }
 
 int hbsa_block_decisions(const hbsa_forward_args* args, uint8_t* decisions, int32_t* counts, void* stream_) {

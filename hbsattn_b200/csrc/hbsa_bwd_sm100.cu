@@ -780,7 +780,8 @@ template <int D, bool BF16, bool KV>
 cudaError_t launch_one(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& x, const CUtensorMap& y, const BwdParams& P, cudaStream_t stream) {
   constexpr size_t smem = 4u * 128u * D * 2u + 2u * kBwdStages * kBwdTile * D * 2u + sizeof(BwdControl);
   static_assert(smem <= 227u * 1024u, "shared memory of one CTA");
-  cudaError_t e = cudaFuncSetAttribute(bwd_sm100_kernel<D, BF16, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static SmemOptIn opt_in;
+  cudaError_t e = opt_in.once(reinterpret_cast<const void*>(bwd_sm100_kernel<D, BF16, KV>), (int)smem);
   if (e != cudaSuccess) return e;
   const long long resident = sm100_sm_count();
   const unsigned grid = (unsigned)(P.total_items < resident ? P.total_items : resident);

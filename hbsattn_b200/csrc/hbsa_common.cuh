@@ -8,11 +8,14 @@
 #include <stddef.h>
 #include <math.h>
 
+#include <atomic>
+
 #include "../../include/hbsattn_b200.h"
 
 namespace hbsa {
 
 constexpr int kStatusWords = 16;
+constexpr int kNotifyWords = 5;      // host words a waiting call reads: tag, then the first status words
 constexpr int kItemWords = 16;       // int32 words of one ItemRecord
 
 // Carved out of the caller's workspace by make_workspace(); every pointer is a device pointer.
@@ -75,10 +78,9 @@ struct RowGeom {
   int n_reach;      // k-blocks [0, n_reach) of the sample can hold a causal-valid element
 };
 
-__device__ __forceinline__ RowGeom row_geometry(const Problem& p, const int32_t* cnq, const int32_t* cnk,
-                                                const int32_t* qb2b, int qb) {
+__device__ __forceinline__ RowGeom row_geometry_of(const Problem& p, const int32_t* cnq, const int32_t* cnk, int b, int qb) {
   RowGeom g;
-  g.b = qb2b[qb];
+  g.b = b;
   const int cq0 = p.cu_q[g.b], cq1 = p.cu_q[g.b + 1];
   const int ck0 = p.cu_k[g.b], ck1 = p.cu_k[g.b + 1];
   g.q_begin = cq0 + (qb - cnq[g.b]) * p.qbs;
@@ -97,6 +99,10 @@ __device__ __forceinline__ RowGeom row_geometry(const Problem& p, const int32_t*
   }
   g.n_reach = reach;
   return g;
+}
+__device__ __forceinline__ RowGeom row_geometry(const Problem& p, const int32_t* cnq, const int32_t* cnk,
+                                                const int32_t* qb2b, int qb) {
+  return row_geometry_of(p, cnq, cnk, qb2b[qb], qb);
 }
 
 // What the attention kernels do when the schedule kernels left an error status: nothing is computed, and the
@@ -134,6 +140,22 @@ __device__ __forceinline__ int sample_of_block(const int32_t* __restrict__ cnb, 
   return lo;
 }
 
+// Raises a kernel's dynamic shared memory limit once per device instead of before every launch (one static object per kernel;
+// racing callers set the same value).
+struct SmemOptIn {
+  std::atomic<unsigned long long> done{0};
+  cudaError_t once(const void* kernel, int bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+};
+
 // printf-style setter of the text hbsa_last_error() returns on the calling thread.
 void set_last_error(const char* fmt, ...);
 
@@ -141,6 +163,13 @@ void set_last_error(const char* fmt, ...);
 cudaError_t launch_calculate_blocks(const int32_t* cu_seqlen, int batch, int block_size, int capacity,
                                     int32_t* cu_block, int32_t* block_to_batch, int32_t* cu_num_block,
                                     cudaStream_t stream);
+// The same tables in one launch for batches it fits (calculate_blocks_fits_one_launch); the number of blocks goes to notify[1] in
+// mapped host memory, then `tag` to notify[0].
+bool calculate_blocks_fits_one_launch(int batch);
+cudaError_t launch_count_and_fill(const int32_t* cu_seqlen, int batch, int block_size, int capacity, int32_t* cu_block,
+                                  int32_t* block_to_batch, int32_t* cu_num_block, int32_t* notify, int tag, cudaStream_t stream);
+// Sends the status words to notify[1..] and `tag` to notify[0] (mapped host memory) when the stream gets there.
+cudaError_t launch_notify(const Workspace& ws, int32_t* notify, int tag, cudaStream_t stream);
 cudaError_t launch_schedule(const Problem& p, const Workspace& ws, uint8_t* decisions, cudaStream_t stream);
 // Rows of one K/V tile the tensor-core kernel uses for k blocks of `kbs` rows.
 int sm100_kv_tile_rows(int kbs);
@@ -162,8 +191,9 @@ int backward_sm100_kv_tile_rows(int kbs);
 int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_backward_args& b, cudaStream_t stream, const char** err_text);
 // Returns nullptr when eligible, else a static string saying why not.
 const char* sm100_ineligible_reason(const hbsa_forward_args& a, float scale);
-// err_text receives a message when a negative HBSA_ERR_* is returned.
+// err_text receives a message when a negative HBSA_ERR_* is returned.  With `notify` (mapped host memory, or NULL) the last CTA to
+// leave sends the status words there, see launch_notify.
 int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forward_args& a,
-                         cudaStream_t stream, const char** err_text);
+                         cudaStream_t stream, int32_t* notify, int tag, const char** err_text);
 
 }  // namespace hbsa

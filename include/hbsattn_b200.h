@@ -4,8 +4,8 @@
  * Every entry point takes plain device pointers, sizes and element strides; no torch
  * types cross this boundary.  All work is enqueued on the CUDA stream passed as the
  * last argument (a cudaStream_t cast to void*; NULL = the legacy default stream) of the
- * device that is current when the call is made.  No entry point synchronises the
- * stream except hbsa_read_status().
+ * device that is current when the call is made.  No entry point waits for the stream except
+ * hbsa_read_status(), hbsa_static_scratch_status(), hbsa_forward_status() and hbsa_calculate_blocks_counted().
  *
  * Return value of every int function: 0 = enqueued; negative = the arguments were
  * rejected before any launch (text in hbsa_last_error()); positive = a CUDA runtime
@@ -76,6 +76,15 @@ int hbsa_calculate_blocks(const int32_t* cu_seqlen, int batch, int block_size, i
                           int32_t* cu_block, int32_t* block_to_batch, int32_t* cu_num_block,
                           void* stream);
 
+/*
+ * The same in one call that waits for the number of blocks: *num_block (host) receives cu_num_block[batch], and the
+ * tables are complete (in stream order) if it does not exceed `capacity`; otherwise only the first `capacity` entries
+ * are, and hbsa_calculate_blocks fills larger arrays.  cu_block and block_to_batch must not be NULL.
+ */
+int hbsa_calculate_blocks_counted(const int32_t* cu_seqlen, int batch, int block_size, int capacity,
+                                  int32_t* cu_block, int32_t* block_to_batch, int32_t* cu_num_block,
+                                  int32_t* num_block, void* stream);
+
 /* Bytes of scratch device memory hbsa_forward / hbsa_block_decisions need for a mask of
  * shape (nhead_k, num_q_block, num_k_block) and `batch` samples.  Depends on nothing else. */
 size_t hbsa_workspace_bytes(int nhead_k, int num_q_block, int num_k_block, int batch);
@@ -141,6 +150,11 @@ typedef struct hbsa_forward_args {
 } hbsa_forward_args;
 
 int hbsa_forward(const hbsa_forward_args* args, void* stream);
+
+/* hbsa_forward that waits until the output is complete and hands back the 16 status words (as hbsa_read_status would, of
+ * which the first four carry information): the kernel itself reports to mapped host memory, which is faster than
+ * hbsa_forward followed by hbsa_read_status. */
+int hbsa_forward_status(const hbsa_forward_args* args, int32_t* status_out, void* stream);
 
 /*
  * The two halves of hbsa_forward, for callers that reuse one mask over several calls (layers,
