@@ -3,6 +3,9 @@
     python hbsattn_b200/build.py [--force] [--verbose] [--strict]
     (run as a script: importing the package needs the library)
 
+Beside the C ABI library it builds _host.so, the CPython extension of csrc/hbsa_host.cpp that the Python operators call into
+(g++ against the headers and libraries of the torch that is installed; no device code).
+
 --strict also builds libhbsattn_b200_strict.so: the same sources with -DHBSA_STRICT_TCGEN05, in which the MMA
 thread of the tensor-core kernel fences after every barrier it observes and waits for the P V products of a lane
 to complete before the next S product overwrites their operand.  It exists to check, bit for bit, the ordering
@@ -18,6 +21,8 @@ import sys
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libhbsattn_b200.so")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "hbsa_host.cpp")
 STRICT_LIB_PATH = os.path.join(PKG_DIR, "libhbsattn_b200_strict.so")
 SOURCES = ["hbsa_api.cu", "hbsa_schedule.cu", "hbsa_fwd_generic.cu", "hbsa_fwd_sm100.cu",
            "hbsa_bwd_sm100.cu", "hbsa_bwd_generic.cu", "hbsa_static_scratch.cu"]
@@ -32,7 +37,7 @@ def _nvcc() -> str:
 
 
 def nvcc_flags(verbose: bool = False):
-    flags = ["-O3", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
+    flags = ["-O3", "--threads", "8", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
              "-Xcompiler", "-fPIC", "-I", os.path.join(PKG_DIR, "..", "include")]
     if verbose:
         flags += ["-Xptxas", "-v"]
@@ -49,7 +54,8 @@ def is_stale(path: str = LIB_PATH) -> bool:
 
 def build(force: bool = False, verbose: bool = False, strict: bool = False) -> str:
     """Compile every CUDA source into hbsattn_b200/libhbsattn_b200.so (or, with strict=True, into
-    libhbsattn_b200_strict.so with -DHBSA_STRICT_TCGEN05); returns the path."""
+    libhbsattn_b200_strict.so with -DHBSA_STRICT_TCGEN05), and the host extension; returns the library's path."""
+    build_host(force)
     out = STRICT_LIB_PATH if strict else LIB_PATH
     if not force and not is_stale(out):
         return out
@@ -61,6 +67,28 @@ def build(force: bool = False, verbose: bool = False, strict: bool = False) -> s
     if res.returncode != 0:
         raise RuntimeError("nvcc failed building %s (exit %d)" % (os.path.basename(out), res.returncode))
     return out
+
+
+def build_host(force: bool = False) -> str:
+    """Compile csrc/hbsa_host.cpp into hbsattn_b200/_host.so; returns the path."""
+    deps = [HOST_SOURCE, os.path.join(PKG_DIR, "..", "include", "hbsattn_b200.h"), os.path.abspath(__file__)]
+    if not force and os.path.exists(HOST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_PATH) for d in deps):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    libs = ["torch_python", "torch", "torch_cpu", "torch_cuda", "c10", "c10_cuda"]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-o", HOST_PATH, HOST_SOURCE, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [f"-I{d}" for d in include] + [f"-L{os.path.join(root, 'lib')}"] + [f"-l{n}" for n in libs]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed building _host.so (exit %d)" % res.returncode)
+    return HOST_PATH
 
 
 if __name__ == "__main__":

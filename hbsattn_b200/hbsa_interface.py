@@ -18,6 +18,7 @@ _DTYPES = {torch.bfloat16: _lib.HBSA_DTYPE_BF16, torch.float16: _lib.HBSA_DTYPE_
 _IMPLS = {"auto": _lib.HBSA_IMPL_AUTO, "generic": _lib.HBSA_IMPL_GENERIC, "sm100": _lib.HBSA_IMPL_SM100}
 
 _state = {"impl": os.environ.get("HBSATTN_B200_IMPL", "auto"), "last_workspace": None}
+_host = _lib.load_host(_state)      # native path of the plain calls; every function of it returns None for what it does not take
 
 
 def set_kernel_family(name: str) -> None:
@@ -148,22 +149,28 @@ class _HBSAttentionFunction(torch.autograd.Function):
         assert q_block_size % 16 == 0 and k_block_size % 16 == 0 and q_block_size > 0 and k_block_size > 0, \
             "q_block_size and k_block_size must be integer multiples of 16."
 
+        want_grad = any(ctx.needs_input_grad[:3])
         cu_q32, cu_k32 = _prepare(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask)
+        if want_grad:
+            ctx.hbsa = (int(q_block_size), int(k_block_size), bool(causal), softmax_scale, int(num_q_block), int(num_k_block))
+            # the backward starts from the log-sum-exp of every row
+            pair = _host.forward(q, k, v, cu_q32, cu_k32, block_mask, q_block_size, k_block_size, causal, softmax_scale, None, None,
+                                 None, None, True, not have_meta and _validate_default())
+            if pair is not None:
+                ctx.save_for_backward(q, k, v, pair[0], pair[1], cu_q32, cu_k32, block_mask)
+                return pair[0]
         lib = _lib.load()
         dev = q.device
-        want_grad = any(ctx.needs_input_grad[:3])
         with torch.cuda.device(dev):
             out = torch.empty(q.shape, dtype=q.dtype, device=dev)
             if q.shape[0] == 0:
                 return out
             ws = alloc_workspace(k.shape[1], num_q_block, num_k_block, cu_q32.numel() - 1, dev)
-            # the backward starts from the log-sum-exp of every row: keep it when a gradient is wanted
             lse = torch.empty((q.shape[0], q.shape[1]), dtype=torch.float32, device=dev) if want_grad else None
             args = make_args(q, k, v, out, cu_q32, cu_k32, block_mask, q_block_size, k_block_size, causal, softmax_scale,
                              num_q_block, num_k_block, ws, _IMPLS[_state["impl"]], lse=lse)
             if want_grad:
                 ctx.save_for_backward(q, k, v, out, lse, cu_q32, cu_k32, block_mask)
-                ctx.hbsa = (int(q_block_size), int(k_block_size), bool(causal), softmax_scale, int(num_q_block), int(num_k_block))
             stream = torch.cuda.current_stream(dev).cuda_stream
             rc = lib.hbsa_forward(ctypes.byref(args), stream)
             if rc != 0:
@@ -189,7 +196,12 @@ class _HBSAttentionFunction(torch.autograd.Function):
         return (dq, dk, dv) + (None,) * 16
 
 
-HBSAttention = _HBSAttentionFunction.apply
+def HBSAttention(*args):
+    """``HBSAttention(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask, q_block_size, k_block_size, causal, softmax_scale,
+    tile_mode='auto', <the eight outputs of calculate_blocks for q and for k>)``, positional as in the reference (see
+    ``_HBSAttentionFunction.forward`` for the arguments).  Calls that record no gradient take the native path."""
+    out = _host.attention(*args)
+    return _HBSAttentionFunction.apply(*args) if out is None else out
 
 
 def attention_backward(q, k, v, out, lse, d_out, cu_q_seqlens, cu_k_seqlens, block_mask, q_block_size, k_block_size, causal,
@@ -203,6 +215,10 @@ def attention_backward(q, k, v, out, lse, d_out, cu_q_seqlens, cu_k_seqlens, blo
         d_out = d_out.to(q.dtype)
     if d_out.stride(2) != 1 or any(n <= 0 or n % 8 for n in d_out.stride()[:2]):
         d_out = d_out.contiguous()                   # an expanded or transposed gradient: the tensor-core kernel loads 16-byte rows
+    if num_q_block in (None, block_mask.shape[1]) and num_k_block in (None, block_mask.shape[2]):
+        grads = _host.backward(q, k, v, cu_q32, cu_k32, block_mask, q_block_size, k_block_size, causal, softmax_scale, out, lse, d_out)
+        if grads is not None:
+            return grads
     nqb = block_mask.shape[1] if num_q_block is None else num_q_block
     nkb = block_mask.shape[2] if num_k_block is None else num_k_block
     lib = _lib.load()
@@ -272,6 +288,10 @@ def HBSAttention_csr(q, k, v, cu_q_seqlens, cu_k_seqlens, csr_row_ptr, csr_col_i
     assert q.shape[1] % k.shape[1] == 0, "nhead_q must be divisible by nhead_k (for GQA)"
     assert q_block_size % 16 == 0 and k_block_size % 16 == 0 and q_block_size > 0 and k_block_size > 0, \
         "q_block_size and k_block_size must be integer multiples of 16."
+    pair = _host.forward(q, k, v, cu_q_seqlens, cu_k_seqlens, None, q_block_size, k_block_size, causal, softmax_scale, csr_row_ptr,
+                         csr_col_idx, num_q_block, num_k_block, False, _validate_default())
+    if pair is not None:
+        return pair[0]
     cu_q32, cu_k32 = _prepare(q, k, v, cu_q_seqlens, cu_k_seqlens, csr_row_ptr)
     row_ptr, col_idx = _check_csr(csr_row_ptr, csr_col_idx, k.shape[1], num_q_block)
     lib = _lib.load()
@@ -363,6 +383,10 @@ def attention_with_schedule(q, k, v, schedule: MaskSchedule, softmax_scale=None)
     assert q.shape[1] % k.shape[1] == 0, "nhead_q must be divisible by nhead_k (for GQA)"
     assert k.shape[1] == schedule.nhead_k, "k has a different number of heads than the schedule's block_mask"
     s = schedule
+    out = _host.scheduled(q, k, v, s.cu_q_seqlens, s.cu_k_seqlens, s.block_mask, s.q_block_size, s.k_block_size, s.causal, softmax_scale,
+                          s.workspace)
+    if out is not None:
+        return out
     _prepare(q, k, v, s.cu_q_seqlens, s.cu_k_seqlens, s.block_mask)
     lib = _lib.load()
     dev = q.device
@@ -391,6 +415,10 @@ def HBSAttention_with_lse(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask, q_blo
     assert q.shape[1] % k.shape[1] == 0, "nhead_q must be divisible by nhead_k (for GQA)"
     assert q_block_size % 16 == 0 and k_block_size % 16 == 0 and q_block_size > 0 and k_block_size > 0, \
         "q_block_size and k_block_size must be integer multiples of 16."
+    pair = _host.forward(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask, q_block_size, k_block_size, causal, softmax_scale, None, None,
+                         None, None, True, _validate_default())
+    if pair is not None:
+        return pair
     cu_q32, cu_k32 = _prepare(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask)
     lib = _lib.load()
     dev = q.device

@@ -1,11 +1,12 @@
 """Block metadata of a packed varlen batch - same name, arguments and return value as the
-reference's ``hbsattn/utils.py:7-50`` (``calculate_blocks``), built by two CUDA kernels through
-the C ABI instead of a dozen torch launches."""
+reference's ``hbsattn/utils.py:7-50`` (``calculate_blocks``), built by CUDA kernels through the
+C ABI instead of a dozen torch launches."""
 from __future__ import annotations
 
 import torch
 
 from . import _lib
+from .hbsa_interface import _host
 
 
 def _calculate_blocks_host(cu_seqlen: torch.Tensor, block_size: int):
@@ -36,6 +37,9 @@ def calculate_blocks(cu_seqlen: torch.Tensor, block_size: int):
     * ``block_to_batch`` int32 ``[num_block]`` sample index of every block
     * ``cu_num_block``   ``[batch+1]`` first block index of every sample, in ``cu_seqlen``'s dtype
     """
+    tables = _host.calculate_blocks(cu_seqlen, block_size)      # one kernel and one wait; None for what it does not take
+    if tables is not None:
+        return tables
     assert cu_seqlen.ndim == 1 and cu_seqlen.numel() >= 2, "cu_seqlen must be a 1D tensor of length batch + 1"
     block_size = int(block_size)
     assert block_size > 0, "block_size must be positive"
