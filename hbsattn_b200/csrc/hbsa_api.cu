@@ -63,7 +63,8 @@ int make_problem(const hbsa_forward_args* a, bool need_tensors, hbsa::Problem* p
   p->kbs = a->k_block_size;
   p->causal = a->causal ? 1 : 0;
   p->scale = a->use_default_scale ? 1.0f / sqrtf((float)a->headdim) : a->softmax_scale;
-  p->kv_tile = hbsa::sm100_kv_tile_rows(a->k_block_size);
+  p->kv_tile = hbsa::kFwdTileRows;
+  p->kv_unit = hbsa::kFwdUnitRows;
   return 0;
 }
 
@@ -279,7 +280,10 @@ int hbsa_backward(const hbsa_backward_args* b, void* stream_) {
     return HBSA_ERR_UNSUPPORTED;
   }
   const bool sm100 = !why && b->fwd.impl != HBSA_IMPL_GENERIC;
-  if (sm100) p.kv_tile = hbsa::backward_sm100_kv_tile_rows(p.kbs);
+  if (sm100) {
+    p.kv_tile = hbsa::backward_sm100_kv_tile_rows(p.kbs);
+    p.kv_unit = 0;
+  }
   cudaError_t e = hbsa::launch_schedule(p, ws, nullptr, stream);
   if (e != cudaSuccess) return fail_cuda(e, "hbsa_backward (schedule)");
   if (sm100) {

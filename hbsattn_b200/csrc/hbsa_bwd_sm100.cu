@@ -376,7 +376,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const int pos = __ffs(bal) - 1;
             bal &= bal - 1;
             const int blk0 = __shfl_sync(0xffffffffu, val, pos) * p.kbs;
-            const int k_end = min(blk0 + p.kbs, rec.k_len);
+            const int k_end = min(blk0 + p.kbs, rec.k_stop);
             for (int k0 = blk0; k0 < k_end && ok; k0 += nt) load_tile(rec.k_begin + k0, rec.hk, nt, k0, k_end);
           }
         }

@@ -41,7 +41,8 @@ struct __align__(16) ItemRecord {
   int q_in0, k_begin, k_len, kb0;    // in-sample index of the first row; the sample's keys and first k-block
   int n_reach, off, n_tiles, count;  // causal-reachable k-blocks, k_len - q_len, K/V tiles to process, active blocks
   int csr_begin;                     // CSR block masks: position in col_idx of the row's first active, reachable entry
-  int pad[3];
+  int k_stop;                        // keys [k_stop, k_len) are out of the q-block's causal reach
+  int pad[2];
 };
 static_assert(sizeof(ItemRecord) == kItemWords * 4, "ItemRecord layout");
 
@@ -61,7 +62,8 @@ struct Problem {
   int num_q_block, num_k_block, qbs, kbs;
   int causal;
   float scale;                          // softmax scale (natural-log domain)
-  int kv_tile;                          // rows of one K/V tile of the tensor-core kernel (0: one tile per k-block)
+  int kv_tile;                          // rows of one K/V tile of the tensor-core kernel that uses the schedule
+  int kv_unit;                          // > 0: its tiles are strung together from pieces of this many rows across the active blocks
 };
 
 // Geometry of one (q-block, sample) pair, derived on the device from cu_seqlens only.
@@ -75,6 +77,7 @@ struct RowGeom {
   int kb0;          // first k-block of the sample (global block index)
   int nkb;          // k-blocks in the sample
   int off;          // k_len - q_len (bottom-right causal alignment)
+  int k_stop;       // keys [0, k_stop) of the sample are causal-valid for its last row
   int n_reach;      // k-blocks [0, n_reach) of the sample can hold a causal-valid element
 };
 
@@ -92,10 +95,12 @@ __device__ __forceinline__ RowGeom row_geometry_of(const Problem& p, const int32
   g.nkb = cnk[g.b + 1] - g.kb0;
   g.off = g.k_len - (cq1 - cq0);
   int reach = g.nkb;
+  g.k_stop = g.k_len;
   if (p.causal) {
     // last row of the q-block, bottom-right aligned: key index it may see at most
     const int limit = (g.q_end - 1 - cq0) + g.off;
     reach = limit < 0 ? 0 : min(g.nkb, limit / p.kbs + 1);
+    g.k_stop = max(0, min(g.k_len, limit + 1));
   }
   g.n_reach = reach;
   return g;
@@ -171,8 +176,8 @@ cudaError_t launch_count_and_fill(const int32_t* cu_seqlen, int batch, int block
 // Sends the status words to notify[1..] and `tag` to notify[0] (mapped host memory) when the stream gets there.
 cudaError_t launch_notify(const Workspace& ws, int32_t* notify, int tag, cudaStream_t stream);
 cudaError_t launch_schedule(const Problem& p, const Workspace& ws, uint8_t* decisions, cudaStream_t stream);
-// Rows of one K/V tile the tensor-core kernel uses for k blocks of `kbs` rows.
-int sm100_kv_tile_rows(int kbs);
+// K/V tiles of the tensor-core forward: 64 rows, strung together from pieces of 16 (blocks of 64 n rows: the same thing).
+constexpr int kFwdTileRows = 64, kFwdUnitRows = 16;
 // Debugging aid: clock budget of every wait inside the tensor-core kernel (<= 0: the default), and a mode in
 // which its producer warp publishes nothing, so that every other wait of the kernel runs out.
 void sm100_set_wait_budget(long long clocks, int stall_producer);

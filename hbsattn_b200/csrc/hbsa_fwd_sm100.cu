@@ -11,7 +11,7 @@
 //    two-slot ring in shared memory and runs ahead of them.  Two CTAs per SM mean two independent
 //    items in flight, so the start and the end of one item hide behind the tiles of the other.
 //  * Only mask-active k-blocks are touched: the producer warp compacts the mask row with warp
-//    ballots and issues TMA loads of exactly those K/V tiles (at most 64 rows each) into two-stage K
+//    ballots and issues TMA loads of exactly those K/V tiles (64 rows each) into two-stage K
 //    and V rings (the reference loops over all k-blocks of the sample and polls the mask byte,
 //    fwd_triton_fix_tile_size.py:117-124).
 //  * S = Q K^T and O += P V are tcgen05.mma instructions with fp32 accumulators in TMEM.  S is
@@ -25,7 +25,7 @@
 //    twelve instructions of a 64-row tile occupy it for as long as the products of both resident CTAs occupy the
 //    pipe (measured: about half of the tile period); it looks for new inputs between the two products only,
 //    and its polling loop is kept to one probe per turn.
-//  * Online softmax in registers, one thread per row: tcgen05.ld of the tile's <= 64 columns, in-place
+//  * Online softmax in registers, one thread per row: tcgen05.ld of the tile's 64 columns, in-place
 //    -inf masking on diagonal / ragged tiles, exp2 with the scale folded in, fp32 row sum; no shuffles
 //    and no shared-memory exchange.  The exponentials of a tile run against the reference maximum of the
 //    previous tiles; only when the tile's row sum (which bounds every P of the row) exceeds 2^14 is the row
@@ -64,7 +64,10 @@ constexpr int kThreads = 192;
 constexpr int kSoftmaxWarps = 4;
 constexpr int kProducerWarp = 4;
 constexpr int kMmaWarp = 5;
-constexpr int kTileRowsMax = 64;      // rows of a K/V tile
+constexpr int kTileRows = kFwdTileRows;   // rows of a K/V tile
+constexpr int kUnitRows = kFwdUnitRows;   // rows of the pieces a gathered tile is made of
+constexpr int kTileUnits = kTileRows / kUnitRows;
+constexpr int kNoKey = 0x40000000;        // "first key" of the empty pieces at the end of a row's last gathered tile
 // S0, S1 of 64 columns + O of D columns, rounded up to a power of two
 template <int D> struct TmemCols { static constexpr uint32_t value = D > 128 ? 512u : 256u; };
 constexpr uint32_t kSStride = 64u;    // TMEM columns between the two S buffers
@@ -77,9 +80,7 @@ struct Sm100Params {
   void* o;
   long long o_s0, o_s1;        // elements
   float* lse;                  // NULL or [total_q, nhead_q]: natural-log sum of exponentials per row
-  int total_q;
-  int nt;                      // rows of one K/V tile (multiple of 16, <= 64)
-  int n_sub;                   // K/V tiles per k-block
+  int total_q, total_k;
   int gp, gp_shift;            // q-heads packed into one M tile
   int n_head_sub;              // group / gp
   int tt;                      // tokens per M tile = 128 / gp
@@ -124,7 +125,7 @@ struct __align__(16) Control {
   uint32_t tmem_base;
   int abort_flag;
   unsigned p_count[2];       // arrivals of the softmax warps for the S buffer tile & 1 (never reset: 4 per tile)
-  int tile_k0[4];
+  __align__(16) int tile_keys[4][kTileUnits];   // in-sample key of the tile's first row (gathered tiles: of every piece)
   ItemSlot slot[2];
 };
 
@@ -175,35 +176,32 @@ __device__ __forceinline__ void issue_qk(uint32_t tS, const uint64_t (&qd)[KSTEP
 #pragma unroll
   for (int ks = 1; ks < KSTEPS; ++ks) ptx::mma_ss_c<true>(tS, qd[ks], kd[ks], idesc);
 }
-// N k-steps of O (+)= P V; the first one overwrites O when `first`.
-template <int N>
-__device__ __forceinline__ void issue_pv_n(uint32_t tO, const uint32_t (&pa)[4], const uint64_t (&vd)[4], uint32_t idesc, bool first) {
+// O (+)= P V of one tile; the first product of an item overwrites O.
+__device__ __forceinline__ void issue_pv(uint32_t tO, const uint32_t (&pa)[4], const uint64_t (&vd)[4], uint32_t idesc, bool first) {
   if (first) ptx::mma_ts_c<false>(tO, pa[0], vd[0], idesc);
   else ptx::mma_ts_c<true>(tO, pa[0], vd[0], idesc);
 #pragma unroll
-  for (int ks = 1; ks < N; ++ks) ptx::mma_ts_c<true>(tO, pa[ks], vd[ks], idesc);
-}
-__device__ __forceinline__ void issue_pv(int n, uint32_t tO, const uint32_t (&pa)[4], const uint64_t (&vd)[4], uint32_t idesc, bool first) {
-  switch (n) {
-    case 1: issue_pv_n<1>(tO, pa, vd, idesc, first); break;
-    case 2: issue_pv_n<2>(tO, pa, vd, idesc, first); break;
-    case 3: issue_pv_n<3>(tO, pa, vd, idesc, first); break;
-    default: issue_pv_n<4>(tO, pa, vd, idesc, first); break;
-  }
+  for (int ks = 1; ks < 4; ++ks) ptx::mma_ts_c<true>(tO, pa[ks], vd[ks], idesc);
 }
 
 // TRACE = true is the instantiation that runs while a debug trace buffer is set; the shipped path carries
 // no stamp code at all.
-// NT > 0 fixes the rows of a K/V tile at compile time (the common 64-row case then has no branches on the tile
-// width); NT = 0 reads them from the parameters.
-template <int D, bool BF16, bool TRACE, int NT>
+// GATHER = false: k-blocks that are multiples of 64 rows; a tile is one box of 64 consecutive keys.
+// GATHER = true: any other k-block size.  The keys of a row's active blocks, in pieces of 16, are strung together and cut
+// into tiles of 64, so that a tile may hold the end of one block and the start of the next: the tile period (about
+// 1 900 clocks of mask-independent latency chain) does not shrink with the tile, and even splits gave 16-row tiles for
+// blocks of 16, 80 or 112.  A piece is one TMA box per 64-column panel, each issued by a lane of its own.  Keys still
+// ascend inside a tile, so that the columns a row may see are a prefix of it.  Measured against the even splits: 64x80
+// blocks, fp16, d = 96, 6 ragged samples 401 -> 188 us; 80x48 blocks, d = 128, 16k tokens 7.38 -> 7.10 ms (a quarter fewer tiles, each
+// of them wider: that shape runs at the 64-row tiles' own pace now).
+template <int D, bool BF16, bool TRACE, bool GATHER>
 __global__ void __launch_bounds__(kThreads, 2)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const Sm100Params P) {
   using namespace ptx;
   constexpr int PANELS = D / 64;
   constexpr uint32_t Q_BYTES = 128u * D * 2u;
-  constexpr uint32_t KV_BYTES_MAX = (uint32_t)kTileRowsMax * D * 2u;
+  constexpr uint32_t KV_BYTES = (uint32_t)kTileRows * D * 2u;
   const Problem& p = P.p;
   using OutT = typename std::conditional<BF16, __nv_bfloat16, __half>::type;
   OutT* const o_base = static_cast<OutT*>(P.o);
@@ -226,15 +224,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   uint8_t* const smem = smem_raw + pad;
   const uint32_t sQ = raw_addr + pad;
   const uint32_t sK = sQ + Q_BYTES;                   // 2 stages
-  const uint32_t sV = sK + 2 * KV_BYTES_MAX;          // 2 stages
-  Control* const ctl = reinterpret_cast<Control*>(smem + Q_BYTES + 4 * KV_BYTES_MAX);
+  const uint32_t sV = sK + 2 * KV_BYTES;          // 2 stages
+  Control* const ctl = reinterpret_cast<Control*>(smem + Q_BYTES + 4 * KV_BYTES);
   const uint32_t bar_item_full = smem_u32(&ctl->item_full[0]), bar_item_done = smem_u32(&ctl->item_done[0]);
   const uint32_t bar_q_full = smem_u32(&ctl->q_full[0]), bar_k_full = smem_u32(&ctl->k_full[0]);
   const uint32_t bar_v_full = smem_u32(&ctl->v_full[0]), bar_s_full = smem_u32(&ctl->s_full[0]);
   const uint32_t bar_pv_done = smem_u32(&ctl->pv_done[0]);
   const uint32_t bar_o_free = smem_u32(&ctl->o_free[0]);
   volatile int* const abort_flag = &ctl->abort_flag;
-  volatile int* const tile_k0 = ctl->tile_k0;
   volatile ItemSlot* const slots = ctl->slot;
 
   if (tid == 0) {
@@ -270,9 +267,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const bool consistent = *(volatile int32_t*)&P.ws.status[0] == HBSA_STATUS_OK;
   const uint32_t tmem_base = ctl->tmem_base;
   const long long budget = P.wait_budget;
-  const int nt = NT > 0 ? NT : P.nt;
-  const uint32_t kv_tile_bytes = (uint32_t)nt * D * 2u;
-  const uint32_t kv_panel_bytes = (uint32_t)nt * 128u;
+  constexpr uint32_t KV_PANEL = (uint32_t)kTileRows * 128u;
 
   if (!consistent) {
     zero_fill_output(o_base, P.o_s0, P.o_s1, 1ll, P.total_q, p.nhead_q, p.headdim, P.lse);
@@ -286,6 +281,44 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     long long next_idx = 0;
     if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
     next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
+    // K and V of tile T into stage T & 1; `key`: the tile's first key (gathered: lane u's is that of piece u)
+    auto load_tile = [&](const ItemRecord& rec, int key) {
+      if (T >= 2) ok = warp_wait(bar_of(bar_s_full, T), par_of(T - 2), abort_flag, budget);
+      if (!ok) return;
+      // where this lane's box starts: its piece (pieces without keys read past the tensor, which TMA fills with zeros) and panel
+      const int unit = lane % kTileUnits, panel = lane / kTileUnits;
+      const int unit_key = GATHER ? __shfl_sync(0xffffffffu, key, unit) : 0;
+      const int unit_row = unit_key == kNoKey ? P.total_k : rec.k_begin + unit_key;
+      if (GATHER ? lane < kTileUnits : lane == 0) *(volatile int*)&ctl->tile_keys[T & 3][lane] = key;
+      __threadfence_block();
+      if (GATHER) __syncwarp();
+      if (lane == 0) mbar_arrive_expect_tx(bar_of(bar_k_full, T), KV_BYTES);
+      if (GATHER) {
+        __syncwarp();
+        if (panel < PANELS)
+          tma_load_3d(sK + (T & 1) * KV_BYTES + panel * KV_PANEL + unit * (kUnitRows * 128u), &tm_k, bar_of(bar_k_full, T), panel * 64, rec.hk, unit_row);
+      } else if (lane == 0) {
+#pragma unroll
+        for (int pn = 0; pn < PANELS; ++pn)
+          tma_load_3d(sK + (T & 1) * KV_BYTES + pn * KV_PANEL, &tm_k, bar_of(bar_k_full, T), pn * 64, rec.hk, rec.k_begin + key);
+      }
+      if (TRACE && lane == 0) stamp(P.trace, T, 0);
+      // V stage T & 1 is free once the P V product of tile T-2 is done
+      if (T >= 2) ok = warp_wait(bar_of(bar_pv_done, T), par_of(T - 2), abort_flag, budget);
+      if (!ok) return;
+      if (lane == 0) mbar_arrive_expect_tx(bar_of(bar_v_full, T), KV_BYTES);
+      if (GATHER) {
+        __syncwarp();
+        if (panel < PANELS)
+          tma_load_3d(sV + (T & 1) * KV_BYTES + panel * KV_PANEL + unit * (kUnitRows * 128u), &tm_v, bar_of(bar_v_full, T), panel * 64, rec.hk, unit_row);
+      } else if (lane == 0) {
+#pragma unroll
+        for (int pn = 0; pn < PANELS; ++pn)
+          tma_load_3d(sV + (T & 1) * KV_BYTES + pn * KV_PANEL, &tm_v, bar_of(bar_v_full, T), pn * 64, rec.hk, rec.k_begin + key);
+      }
+      if (TRACE && lane == 0) stamp(P.trace, T, 1);
+      ++T;
+    };
     while (ok) {
       const long long idx = next_idx;
       const bool have = idx < P.total_items;
@@ -340,7 +373,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const uint8_t* mrow = csr ? nullptr : p.mask + rec.hk * p.mask_s0 + rec.qb * p.mask_s1 + (long long)rec.kb0 * p.mask_s2;
       const int32_t* cidx = csr ? p.csr_idx + rec.csr_begin : nullptr;
       bool bit_next = false;
-      int val_next = 0;
+      int val_next = 0, fill = 0, unit_key = 0;
       if (csr) val_next = lane < n_src ? cidx[lane] - rec.kb0 : 0;
       else bit_next = lane < n_src && mrow[(long long)lane * p.mask_s2] != 0;
       for (int base = 0; base < n_src && ok; base += 32) {
@@ -360,36 +393,27 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         while (bal != 0 && ok) {
           const int pos = __ffs(bal) - 1;
           bal &= bal - 1;
-          const int jj = csr ? __shfl_sync(0xffffffffu, val_cur, pos) : base + pos;
-          const int blk_k0 = jj * p.kbs;
-          for (int sub = 0; sub < P.n_sub && ok; ++sub) {
-            const int k0 = blk_k0 + sub * nt;
-            if (k0 >= rec.k_len) break;
-            if (T >= 2) ok = warp_wait(bar_of(bar_s_full, T), par_of(T - 2), abort_flag, budget);
-            if (!ok) break;
-            if (lane == 0) {
-              tile_k0[T & 3] = k0;
-              __threadfence_block();
-              mbar_arrive_expect_tx(bar_of(bar_k_full, T), kv_tile_bytes);
-#pragma unroll
-              for (int pn = 0; pn < PANELS; ++pn)
-                tma_load_3d(sK + (T & 1) * KV_BYTES_MAX + pn * kv_panel_bytes, &tm_k, bar_of(bar_k_full, T), pn * 64, rec.hk, rec.k_begin + k0);
-              if (TRACE) stamp(P.trace, T, 0);
+          const int blk_k0 = (csr ? __shfl_sync(0xffffffffu, val_cur, pos) : base + pos) * p.kbs;
+          const int blk_end = min(blk_k0 + p.kbs, rec.k_stop);
+          if (!GATHER) {
+            for (int k0 = blk_k0; k0 < blk_end && ok; k0 += kTileRows) load_tile(rec, k0);
+          } else {
+            // lane u < kTileUnits holds the first key of the open tile's piece u
+            for (int k0 = blk_k0; k0 < blk_end && ok;) {
+              const int key = k0 + (lane - fill) * kUnitRows;
+              if (lane >= fill && key < blk_end) unit_key = key;
+              const int take = min(kTileUnits - fill, (blk_end - k0 + kUnitRows - 1) / kUnitRows);
+              k0 += take * kUnitRows;
+              fill += take;
+              if (fill == kTileUnits) {
+                load_tile(rec, unit_key);
+                fill = 0;
+              }
             }
-            // V stage T & 1 is free once the P V product of tile T-2 is done
-            if (T >= 2) ok = warp_wait(bar_of(bar_pv_done, T), par_of(T - 2), abort_flag, budget);
-            if (!ok) break;
-            if (lane == 0) {
-              mbar_arrive_expect_tx(bar_of(bar_v_full, T), kv_tile_bytes);
-#pragma unroll
-              for (int pn = 0; pn < PANELS; ++pn)
-                tma_load_3d(sV + (T & 1) * KV_BYTES_MAX + pn * kv_panel_bytes, &tm_v, bar_of(bar_v_full, T), pn * 64, rec.hk, rec.k_begin + k0);
-              if (TRACE) stamp(P.trace, T, 1);
-            }
-            ++T;
           }
         }
       }
+      if (GATHER && fill > 0 && ok) load_tile(rec, lane < fill ? unit_key : kNoKey);
     }
     if (!ok) {
       // Gave up: let the copies already issued land before the CTA retires (bounded).
@@ -406,11 +430,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // S(t+2) writes.  The thread polls with non-blocking probes and issues whichever of "next P V" / "next
     // S" has its inputs ready; a clock budget bounds the loop.
     if (lane == 0) {
-      const uint32_t idesc_qk = make_idesc(BF16, false, false, 128, nt);
+      const uint32_t idesc_qk = make_idesc(BF16, false, false, 128, kTileRows);
       const uint32_t idesc_pv = make_idesc(BF16, false, true, 128, D);
-      const int ksteps = nt >> 4;
       const uint32_t desc_hi = smem_desc_hi(1024u);
-      const uint32_t kpanel_units = kv_panel_bytes >> 4;
+      const uint32_t kpanel_units = KV_PANEL >> 4;
       // Q and K are K-major: 16 head dims further = 32 bytes = 2 descriptor units inside a 64-dim panel.
       // V is MN-major: 16 keys further = 2048 bytes = 128 units.  P: 8 TMEM columns per 16 keys.
       uint64_t qd[D / 16], kd0[D / 16], kd1[D / 16], vd0[4], vd1[4];
@@ -421,12 +444,12 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         const uint32_t qo = (uint32_t)(ks >> 2) * 1024u + (uint32_t)(ks & 3) * 2u;
         qd[ks] = smem_desc_join(smem_desc_lo(sQ, 16u) + qo, desc_hi);
         kd0[ks] = smem_desc_join(smem_desc_lo(sK, 16u) + ko, desc_hi);
-        kd1[ks] = smem_desc_join(smem_desc_lo(sK + KV_BYTES_MAX, 16u) + ko, desc_hi);
+        kd1[ks] = smem_desc_join(smem_desc_lo(sK + KV_BYTES, 16u) + ko, desc_hi);
       }
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
-        vd0[ks] = smem_desc_join(smem_desc_lo(sV, kv_panel_bytes) + (uint32_t)ks * 128u, desc_hi);
-        vd1[ks] = smem_desc_join(smem_desc_lo(sV + KV_BYTES_MAX, kv_panel_bytes) + (uint32_t)ks * 128u, desc_hi);
+        vd0[ks] = smem_desc_join(smem_desc_lo(sV, KV_PANEL) + (uint32_t)ks * 128u, desc_hi);
+        vd1[ks] = smem_desc_join(smem_desc_lo(sV + KV_BYTES, KV_PANEL) + (uint32_t)ks * 128u, desc_hi);
         pa0[ks] = tmem_base + (uint32_t)ks * 8u;
         pa1[ks] = tmem_base + kSStride + (uint32_t)ks * 8u;
       }
@@ -481,8 +504,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             tc_fence_after();
 #endif
             if (TRACE) stamp(P.trace, pT, 4);
-            if (pT & 1) issue_pv(ksteps, tO, pa1, vd1, idesc_pv, (fl & 1) != 0);
-            else issue_pv(ksteps, tO, pa0, vd0, idesc_pv, (fl & 1) != 0);
+            if (pT & 1) issue_pv(tO, pa1, vd1, idesc_pv, (fl & 1) != 0);
+            else issue_pv(tO, pa0, vd0, idesc_pv, (fl & 1) != 0);
             tc_commit(bar_of(bar_pv_done, pT));
             if (TRACE) stamp(P.trace, pT, 5);
             if (fl & 1) ++pIq;
@@ -541,7 +564,6 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // =============================== softmax + epilogue ===============================
     const int row = tid;                             // 0..127: row of the M tile = TMEM lane
     const uint32_t lane_off = (uint32_t)(warp * 32) << 16;
-    const int my_nc = nt;                            // columns of a tile: 16, 32, 48 or 64
     const uint32_t tOmine = tmem_base + kTmemOCol + lane_off;
     const float scale_log2 = P.scale_log2;
     int I = 0, Iq = 0, T = 0;
@@ -572,18 +594,26 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (!ok) break;
           tc_fence_after();
           if (TRACE && tid == 0) stamp(P.trace, T, 6);
-          const int col_limit = limit_row - tile_k0[T & 3];            // tile columns <= col_limit are valid
+          int col_limit;                                 // tile columns <= col_limit are valid
+          if (GATHER) {
+            col_limit = -1;
+#pragma unroll
+            for (int u = 0; u < kTileUnits; ++u)
+              col_limit += min(max(limit_row + 1 - *(volatile int*)&ctl->tile_keys[T & 3][u], 0), kUnitRows);
+          } else {
+            col_limit = limit_row - *(volatile int*)&ctl->tile_keys[T & 3][0];
+          }
           const uint32_t tSmine = tmem_base + (uint32_t)(T & 1) * kSStride + lane_off;
 
           // ---- this thread's row of S, all in registers.  The first 16 columns are awaited alone so that
           //      work on them overlaps the TMEM latency of the rest.
           uint32_t r[64];
-          const bool edge = col_limit < my_nc - 1;      // tile on the causal diagonal or at the ragged end of the sample
+          const bool edge = col_limit < kTileRows - 1;      // tile on the causal diagonal or at the ragged end of the sample
           tmem_ld16(tSmine, *reinterpret_cast<uint32_t(*)[16]>(&r[0]));
           tmem_wait_ld();
 #pragma unroll
           for (int j = 1; j < 4; ++j)
-            if (my_nc > 16 * j) tmem_ld16(tSmine + 16 * j, *reinterpret_cast<uint32_t(*)[16]>(&r[16 * j]));
+            tmem_ld16(tSmine + 16 * j, *reinterpret_cast<uint32_t(*)[16]>(&r[16 * j]));
           if (TRACE && tid == 0) stamp(P.trace, T, 12);
 
           float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -594,36 +624,31 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             // gives the same softmax; the reference only has to keep P in range).  If the tile turns out to be
             // out of range, the exact pass below redoes it.
             const float neg_m0 = m_ref == -INFINITY ? 0.f : -m_ref;
-            // With the tile width fixed at compile time, tiles without masked columns (all but those on the causal
-            // diagonal or at the ragged end of a sample) take a copy of the loop that has no per-group branch; the
-            // test is warp-uniform because the TMEM stores are warp-wide instructions.
-            if (NT > 0 && !__any_sync(0xffffffffu, edge)) {
+            // Tiles without masked columns (all but those on the causal diagonal or at the end of a row's keys) take a
+            // copy of the loop that has no per-group branch; the test is warp-uniform because the TMEM stores are
+            // warp-wide instructions.
+            if (!__any_sync(0xffffffffu, edge)) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                if (my_nc > 16 * j) {
-                  if (j == 1) tmem_wait_ld();
-                  uint32_t pk[8];
-                  exp16<BF16>(&r[16 * j], pk, scale_log2, neg_m0, sum);
-                  tmem_st8(tSmine + 8 * j, pk);
-                }
+                if (j == 1) tmem_wait_ld();
+                uint32_t pk[8];
+                exp16<BF16>(&r[16 * j], pk, scale_log2, neg_m0, sum);
+                tmem_st8(tSmine + 8 * j, pk);
               }
             } else {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                if (my_nc > 16 * j) {
-                  if (j == 1) tmem_wait_ld();
-                  if (edge) {
+                if (j == 1) tmem_wait_ld();
+                if (edge) {
 #pragma unroll
-                    for (int i = 16 * j; i < 16 * j + 16; ++i)
-                      if (i > col_limit) r[i] = 0xff800000u;               // -inf: exp2 makes it an exact 0
-                  }
-                  uint32_t pk[8];
-                  exp16<BF16>(&r[16 * j], pk, scale_log2, neg_m0, sum);
-                  tmem_st8(tSmine + 8 * j, pk);
+                  for (int i = 16 * j; i < 16 * j + 16; ++i)
+                    if (i > col_limit) r[i] = 0xff800000u;               // -inf: exp2 makes it an exact 0
                 }
+                uint32_t pk[8];
+                exp16<BF16>(&r[16 * j], pk, scale_log2, neg_m0, sum);
+                tmem_st8(tSmine + 8 * j, pk);
               }
             }
-            if (my_nc <= 16) tmem_wait_ld();
             // Whether the reference is stale is read off the tile's row sum, which is there anyway: P >= 0, so no P
             // exceeds it, and a sum of at most 2^14 keeps every P far inside the range of both 16-bit formats (an
             // overflowed exponential makes the sum infinite).  The row maximum itself is only computed on that (rare)
@@ -634,7 +659,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (__any_sync(0xffffffffu, need)) {
 #pragma unroll
               for (int j = 0; j < 4; ++j)
-                if (my_nc > 16 * j) max16(&r[16 * j], mx4);
+                max16(&r[16 * j], mx4);
               const float mx_s = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;   // scale > 0 keeps the order
               need = mx_s > m_ref + kRescaleThreshold;
               if (__any_sync(0xffffffffu, need)) {       // (a row without reference whose tile is all masked needs nothing)
@@ -668,7 +693,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              if (my_nc > 16 * j) max16(&r[16 * j], mx4);
+              max16(&r[16 * j], mx4);
             m_ref = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
             if (TRACE && tid == 0) stamp(P.trace, T, 7);
           }
@@ -677,11 +702,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              if (my_nc > 16 * j) {
-                uint32_t pk[8];
-                exp16<BF16>(&r[16 * j], pk, scale_log2, neg_m, sum);
-                tmem_st8(tSmine + 8 * j, pk);
-              }
+              uint32_t pk[8];
+              exp16<BF16>(&r[16 * j], pk, scale_log2, neg_m, sum);
+              tmem_st8(tSmine + 8 * j, pk);
             }
           }
           l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
@@ -856,13 +879,6 @@ void sm100_set_wait_budget(long long clocks, int stall_producer) {
 void sm100_set_trace(long long* device_buffer) { g_trace = device_buffer; }
 size_t sm100_trace_bytes() { return ((size_t)kTraceTiles * kTraceSlots + 2 * kTraceCtas) * sizeof(long long); }
 
-int sm100_kv_tile_rows(int kbs) {
-  if (kbs <= kTileRowsMax) return kbs;
-  for (int nt = kTileRowsMax; nt >= 16; nt -= 16)
-    if (kbs % nt == 0) return nt;
-  return 16;
-}
-
 const char* sm100_ineligible_reason(const hbsa_forward_args& a, float scale) {
   if (a.dtype != HBSA_DTYPE_BF16 && a.dtype != HBSA_DTYPE_F16) return "dtype is not bf16/fp16";
   if (a.headdim % 8 != 0 || a.headdim < 16 || a.headdim > 256) return "headdim is not a multiple of 8 between 16 and 256";
@@ -893,8 +909,8 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   P.total_q = a.total_q;
   P.o_s0 = a.o_stride[0];
   P.o_s1 = a.o_stride[1];
-  P.nt = sm100_kv_tile_rows(p.kbs);
-  P.n_sub = p.kbs / P.nt;
+  P.total_k = a.total_k;
+  const bool gather = p.kbs % kTileRows != 0;
   int gp = 1;
   while (gp < 128 && p.group % (gp * 2) == 0) gp *= 2;
   P.gp = gp;
@@ -921,8 +937,8 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
 
   CUtensorMap tq, tk, tv;
   if (!sm100_encode_map(fn, &tq, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], gp, P.tt) ||
-      !sm100_encode_map(fn, &tk, bf16, a.k, p.headdim, p.nhead_k, a.total_k, a.k_stride[0], a.k_stride[1], 1, P.nt) ||
-      !sm100_encode_map(fn, &tv, bf16, a.v, p.headdim, p.nhead_k, a.total_k, a.v_stride[0], a.v_stride[1], 1, P.nt)) {
+      !sm100_encode_map(fn, &tk, bf16, a.k, p.headdim, p.nhead_k, a.total_k, a.k_stride[0], a.k_stride[1], 1, gather ? kUnitRows : kTileRows) ||
+      !sm100_encode_map(fn, &tv, bf16, a.v, p.headdim, p.nhead_k, a.total_k, a.v_stride[0], a.v_stride[1], 1, gather ? kUnitRows : kTileRows)) {
     *err_text = "cuTensorMapEncodeTiled rejected a q/k/v layout";
     return HBSA_ERR_UNSUPPORTED;
   }
@@ -931,7 +947,7 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   // innermost extent, the hardware fills those columns of Q, K and V with zeros (so S is exact and the surplus
   // columns of O are zeros), and the epilogue stores the real columns only.
   const int d_tile = p.headdim <= 64 ? 64 : p.headdim <= 128 ? 128 : 256;
-  const size_t smem = (128u + 4u * (size_t)kTileRowsMax) * (size_t)d_tile * 2u + sizeof(Control) + 1024u;
+  const size_t smem = (128u + 4u * (size_t)kTileRows) * (size_t)d_tile * 2u + sizeof(Control) + 1024u;
   cudaError_t e = cudaSuccess;
   // Programmatic launch (2-3 us less between the two kernels of a forward): the CTAs set up barriers and tensor memory while the schedule kernel is still running.
   cudaLaunchAttribute attr;
@@ -944,17 +960,17 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-#define HBSA_LAUNCH_SM100(D_, BF_, TR_, NT_)                                                              \
+#define HBSA_LAUNCH_SM100(D_, BF_, TR_, GA_)                                                              \
   do {                                                                                                   \
     static SmemOptIn opt_in;                                                                             \
-    e = opt_in.once(reinterpret_cast<const void*>(fwd_sm100_kernel<D_, BF_, TR_, NT_>), (int)smem);       \
-    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fwd_sm100_kernel<D_, BF_, TR_, NT_>, tq, tk, tv, P); \
+    e = opt_in.once(reinterpret_cast<const void*>(fwd_sm100_kernel<D_, BF_, TR_, GA_>), (int)smem);       \
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fwd_sm100_kernel<D_, BF_, TR_, GA_>, tq, tk, tv, P); \
   } while (0)
 #define HBSA_LAUNCH_SM100_T(D_, BF_)                                                                      \
   do {                                                                                                   \
-    if (P.trace != nullptr) HBSA_LAUNCH_SM100(D_, BF_, true, 0);                                         \
-    else if (P.nt == 64) HBSA_LAUNCH_SM100(D_, BF_, false, 64);                                          \
-    else HBSA_LAUNCH_SM100(D_, BF_, false, 0);                                                           \
+    if (gather) HBSA_LAUNCH_SM100(D_, BF_, false, true);                                                 \
+    else if (P.trace != nullptr) HBSA_LAUNCH_SM100(D_, BF_, true, false);                                \
+    else HBSA_LAUNCH_SM100(D_, BF_, false, false);                                                       \
   } while (0)
   if (d_tile == 256) { if (bf16) HBSA_LAUNCH_SM100_T(256, true); else HBSA_LAUNCH_SM100_T(256, false); }
   else if (d_tile == 128) { if (bf16) HBSA_LAUNCH_SM100_T(128, true); else HBSA_LAUNCH_SM100_T(128, false); }

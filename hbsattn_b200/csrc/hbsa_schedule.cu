@@ -209,7 +209,7 @@ cudaError_t launch_calculate_blocks(const int32_t* cu_seqlen, int batch, int blo
 __device__ __forceinline__ void count_row(const Problem& p, const Workspace& ws, uint8_t* __restrict__ decisions, const RowGeom& g,
                                           long long row, int hk, int qb, long long pos) {
   const int lane = threadIdx.x & 31;
-  const int j_last = g.nkb - 1;                 // the ragged last k-block of the sample may own fewer tiles
+  const int j_last = g.n_reach - 1;             // the last reachable k-block may own fewer tiles
   int cnt = 0, csr_begin = 0;
   bool last_active = false;
   const uint8_t* mrow = nullptr;
@@ -219,7 +219,7 @@ __device__ __forceinline__ void count_row(const Problem& p, const Workspace& ws,
     csr_begin = lower_bound_i32(p.csr_idx, e0, e1, g.kb0);
     const int hi = lower_bound_i32(p.csr_idx, csr_begin, e1, g.kb0 + g.n_reach);
     cnt = hi - csr_begin;
-    last_active = cnt > 0 && j_last < g.n_reach && p.csr_idx[hi - 1] == g.kb0 + j_last;
+    last_active = cnt > 0 && p.csr_idx[hi - 1] == g.kb0 + j_last;
   } else {
     mrow = p.mask + hk * p.mask_s0 + qb * p.mask_s1;
 #pragma unroll 4
@@ -234,20 +234,20 @@ __device__ __forceinline__ void count_row(const Problem& p, const Workspace& ws,
   }
   if (lane == 0) {
     ws.counts[row] = cnt;
-    int n_tiles = cnt;
-    if (p.kv_tile > 0 && p.kv_tile < p.kbs) {
-      const int n_sub = (p.kbs + p.kv_tile - 1) / p.kv_tile;
-      n_tiles = cnt * n_sub;
-      if (last_active) {
-        const int len_last = g.k_len - j_last * p.kbs;
-        n_tiles -= n_sub - (len_last + p.kv_tile - 1) / p.kv_tile;
-      }
+    // pieces of the row (tiles, where tiles do not cross block boundaries); the last reachable block may own fewer
+    const int piece = p.kv_unit > 0 ? p.kv_unit : p.kv_tile;
+    const int n_sub = (p.kbs + piece - 1) / piece;
+    int n_tiles = cnt * n_sub;
+    if (last_active) n_tiles -= n_sub - (min(g.k_stop - j_last * p.kbs, p.kbs) + piece - 1) / piece;
+    if (p.kv_unit > 0) {
+      const int per_tile = p.kv_tile / p.kv_unit;
+      n_tiles = (n_tiles + per_tile - 1) / per_tile;
     }
     ItemRecord rec;
     rec.hk = hk; rec.qb = qb; rec.q_begin = g.q_begin; rec.q_end = g.q_end;
     rec.q_in0 = g.q_in0; rec.k_begin = g.k_begin; rec.k_len = g.k_len; rec.kb0 = g.kb0;
     rec.n_reach = g.n_reach; rec.off = g.off; rec.n_tiles = n_tiles; rec.count = cnt;
-    rec.csr_begin = csr_begin; rec.pad[0] = rec.pad[1] = rec.pad[2] = 0;
+    rec.csr_begin = csr_begin; rec.k_stop = g.k_stop; rec.pad[0] = rec.pad[1] = 0;
     reinterpret_cast<ItemRecord*>(ws.items)[pos] = rec;
   }
   if (decisions) {
