@@ -37,7 +37,7 @@ def _nvcc() -> str:
 
 
 def nvcc_flags(verbose: bool = False):
-    flags = ["-O3", "--threads", "8", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
+    flags = ["-O3", "--threads", "8", "--split-compile", "8", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
              "-Xcompiler", "-fPIC", "-I", os.path.join(PKG_DIR, "..", "include")]
     if verbose:
         flags += ["-Xptxas", "-v"]

@@ -67,6 +67,8 @@ constexpr int kMmaWarp = 5;
 constexpr int kTileRows = kFwdTileRows;   // rows of a K/V tile
 constexpr int kUnitRows = kFwdUnitRows;   // rows of the pieces a gathered tile is made of
 constexpr int kTileUnits = kTileRows / kUnitRows;
+constexpr int kSplitTiles = 24;           // tiles of a dense row that a CTA of a cluster gets at least
+constexpr size_t kSplitSmem = 80u * 1024u;   // more than a third of an SM's shared memory
 constexpr int kNoKey = 0x40000000;        // "first key" of the empty pieces at the end of a row's last gathered tile
 // S0, S1 of 64 columns + O of D columns, rounded up to a power of two
 template <int D> struct TmemCols { static constexpr uint32_t value = D > 128 ? 512u : 256u; };
@@ -81,6 +83,7 @@ struct Sm100Params {
   long long o_s0, o_s1;        // elements
   float* lse;                  // NULL or [total_q, nhead_q]: natural-log sum of exponentials per row
   int total_q, total_k;
+  int split;                   // CTAs of the cluster that share one work item (1: no cluster)
   int gp, gp_shift;            // q-heads packed into one M tile
   int n_head_sub;              // group / gp
   int tt;                      // tokens per M tile = 128 / gp
@@ -115,18 +118,20 @@ struct ItemSlot {
   int qi0;            // in-sample index of the tile's first token
   int k_len;
   int off;            // k_len - q_len
-  int pad;
+  int item_tiles;     // tiles of the item, over all CTAs that share it
 };
 
 struct __align__(16) Control {
   unsigned long long item_full[2], item_done[2];
   unsigned long long q_full[2], k_full[2], v_full[2], s_full[2], pv_done[2], o_free[2];
   unsigned long long drain;
+  unsigned long long parts_ready;   // SPLIT: the partial results of every CTA of the cluster are in shared memory
   uint32_t tmem_base;
   int abort_flag;
   unsigned p_count[2];       // arrivals of the softmax warps for the S buffer tile & 1 (never reset: 4 per tile)
   __align__(16) int tile_keys[4][kTileUnits];   // in-sample key of the tile's first row (gathered tiles: of every piece)
   ItemSlot slot[2];
+  float2 part_ml[128];       // SPLIT: reference maximum and row sum of this CTA's part
 };
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -194,7 +199,15 @@ __device__ __forceinline__ void issue_pv(uint32_t tO, const uint32_t (&pa)[4], c
 // ascend inside a tile, so that the columns a row may see are a prefix of it.  Measured against the even splits: 64x80
 // blocks, fp16, d = 96, 6 ragged samples 401 -> 188 us; 80x48 blocks, d = 128, 16k tokens 7.38 -> 7.10 ms (a quarter fewer tiles, each
 // of them wider: that shape runs at the 64-row tiles' own pace now).
-template <int D, bool BF16, bool TRACE, bool GATHER>
+//
+// SPLIT = true: launches with fewer items than the chip takes (one new token per sample, a few heads, short prompts).  A cluster
+// of 2, 4 or 8 CTAs shares every item: CTA r takes the tiles r, r + c, ... of the row's list, leaves its unnormalised O in
+// fp32 where its K and V stages were, its maxima and sums beside it, and after one cluster-wide meeting the CTAs write disjoint
+// pieces of the item's output, reading each other's parts through distributed shared memory.  No scratch in global memory, no second
+// kernel.  A CTA works on one item only (the hardware hands out the clusters), so nothing is reused and nobody leaves
+// before the closing cluster barrier.  One token on 16 contexts of 16k to 32k keys, 8 kv-heads, d = 64: 128 items left 20 SMs
+// idle and the others with one CTA each, 125 us; in parts of 2 / 4 / 8: 81 / 83 / 110 us.
+template <int D, bool BF16, bool TRACE, bool GATHER, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 2)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const Sm100Params P) {
@@ -246,6 +259,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_init(bar_o_free + 8 * i, kSoftmaxWarps);
     }
     mbar_init(smem_u32(&ctl->drain), 1);
+    if (SPLIT) mbar_init(smem_u32(&ctl->parts_ready), (uint32_t)(kSoftmaxWarps * P.split));
     ctl->abort_flag = 0;
     ctl->p_count[0] = ctl->p_count[1] = 0u;
     fence_barrier_init();
@@ -260,8 +274,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  if (SPLIT) cluster_sync();                           // the peers' barriers exist before anybody arrives on them
+  else __syncthreads();
   tc_fence_after();
+  const int part = SPLIT ? (int)cluster_ctarank() : 0, parts = SPLIT ? P.split : 1;
   // Everything above overlaps the schedule kernel in front of this launch; from here on its results are needed.
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const bool consistent = *(volatile int32_t*)&P.ws.status[0] == HBSA_STATUS_OK;
@@ -279,7 +295,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     bool ok = P.debug_stall == 0;
     // one fetch ahead: the atomic and the record load of the next item overlap the current item
     long long next_idx = 0;
-    if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
+    if (SPLIT) next_idx = blockIdx.x / (unsigned)parts;
+    else if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
     next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
     // K and V of tile T into stage T & 1; `key`: the tile's first key (gathered: lane u's is that of piece u)
     auto load_tile = [&](const ItemRecord& rec, int key) {
@@ -327,14 +344,15 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (have) {
         rec = records[idx / P.items_per_row];
         rem = (int)(idx % P.items_per_row);
-        if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
+        if (SPLIT) next_idx = P.total_items;
+        else if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
         next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
       }
       const int hsub = rem / P.tiles_per_qblock, qt = rem % P.tiles_per_qblock;
       const int tile_tok0 = rec.q_begin + qt * P.tt;
       if (have && tile_tok0 >= rec.q_end) continue;          // M tile past the ragged end of the q-block
       const int head0 = rec.hk * p.group + hsub * P.gp;
-      const int n_tiles = have ? rec.n_tiles : -1;
+      const int n_tiles = !have ? -1 : SPLIT ? (rec.n_tiles - part + parts - 1) / parts : rec.n_tiles;
 
       // publish: slot I & 1 is free once every consumer has left item I - 2
       if (I >= 2) ok = warp_wait(bar_of(bar_item_done, I), par_of(I - 2), abort_flag, budget);
@@ -348,6 +366,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         sl->qi0 = rec.q_in0 + qt * P.tt;
         sl->k_len = rec.k_len;
         sl->off = rec.off;
+        sl->item_tiles = rec.n_tiles;
         __threadfence_block();
         mbar_arrive(bar_of(bar_item_full, I));
       }
@@ -373,7 +392,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       const uint8_t* mrow = csr ? nullptr : p.mask + rec.hk * p.mask_s0 + rec.qb * p.mask_s1 + (long long)rec.kb0 * p.mask_s2;
       const int32_t* cidx = csr ? p.csr_idx + rec.csr_begin : nullptr;
       bool bit_next = false;
-      int val_next = 0, fill = 0, unit_key = 0;
+      int val_next = 0, fill = 0, unit_key = 0, turn = part;       // turn: tiles of the row until this CTA's next one
       if (csr) val_next = lane < n_src ? cidx[lane] - rec.kb0 : 0;
       else bit_next = lane < n_src && mrow[(long long)lane * p.mask_s2] != 0;
       for (int base = 0; base < n_src && ok; base += 32) {
@@ -396,7 +415,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           const int blk_k0 = (csr ? __shfl_sync(0xffffffffu, val_cur, pos) : base + pos) * p.kbs;
           const int blk_end = min(blk_k0 + p.kbs, rec.k_stop);
           if (!GATHER) {
-            for (int k0 = blk_k0; k0 < blk_end && ok; k0 += kTileRows) load_tile(rec, k0);
+            for (int k0 = blk_k0; k0 < blk_end && ok; k0 += kTileRows) {
+              if (!SPLIT || turn == 0) load_tile(rec, k0);
+              if (SPLIT) turn = turn == 0 ? parts - 1 : turn - 1;
+            }
           } else {
             // lane u < kTileUnits holds the first key of the open tile's piece u
             for (int k0 = blk_k0; k0 < blk_end && ok;) {
@@ -406,14 +428,15 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
               k0 += take * kUnitRows;
               fill += take;
               if (fill == kTileUnits) {
-                load_tile(rec, unit_key);
+                if (!SPLIT || turn == 0) load_tile(rec, unit_key);
+                if (SPLIT) turn = turn == 0 ? parts - 1 : turn - 1;
                 fill = 0;
               }
             }
           }
         }
       }
-      if (GATHER && fill > 0 && ok) load_tile(rec, lane < fill ? unit_key : kNoKey);
+      if (GATHER && fill > 0 && ok && (!SPLIT || turn == 0)) load_tile(rec, lane < fill ? unit_key : kNoKey);
     }
     if (!ok) {
       // Gave up: let the copies already issued land before the CTA retires (bounded).
@@ -568,16 +591,76 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const float scale_log2 = P.scale_log2;
     int I = 0, Iq = 0, T = 0;
     bool ok = true;
+    // SPLIT: this CTA's part of the item to shared memory, then its share of the item's output from all parts
+    auto finish_part = [&](int tile_tok0, int head0, int q_end, float m_ref, float l, int last_tile) -> bool {
+      const int rows = min(P.tt, q_end - tile_tok0) << P.gp_shift;       // rows of the M tile that exist; they come first
+      const uint32_t part_o = sK;                                        // [128][D] fp32 over the K and V stages, 16-byte chunks swizzled
+      if (last_tile >= 0) {
+        if (!warp_wait(bar_of(bar_pv_done, last_tile), par_of(last_tile), abort_flag, budget)) return false;
+        tc_fence_after();
+        if (warp * 32 < rows) {
+#pragma unroll 1
+          for (int c0 = 0; c0 < D; c0 += 32) {
+            uint32_t o[32];
+            tmem_ld32(tOmine + c0, o);
+            tmem_wait_ld();
+            if (row < rows) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                st_shared_v4(part_o + (uint32_t)row * (D * 4u) + (uint32_t)(((c0 >> 2) + i) ^ (row & 7)) * 16u, o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+            }
+          }
+        }
+      }
+      ctl->part_ml[row] = make_float2(m_ref, l);
+      __syncwarp();
+      if (lane < parts) mbar_arrive_cluster(map_to_rank(smem_u32(&ctl->parts_ready), (uint32_t)lane));
+      if (!__all_sync(0xffffffffu, mbar_wait_cluster_bounded(smem_u32(&ctl->parts_ready), 0u, abort_flag, budget))) return false;
+      const int chunks = p.headdim >> 3;
+      const uint32_t ml = smem_u32(&ctl->part_ml[0]);
+      for (int u = part * (kSoftmaxWarps * 32) + tid; u < rows * chunks; u += parts * (kSoftmaxWarps * 32)) {
+        const int r = u / chunks, ch = u - r * chunks;
+        float m = -INFINITY;
+        for (int i = 0; i < parts; ++i) {
+          float mi, li;
+          ld_cluster_v2(map_to_rank(ml + 8u * (uint32_t)r, (uint32_t)i), mi, li);
+          if (li != 0.f) m = fmaxf(m, mi);
+        }
+        float sum = 0.f, acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int i = 0; i < parts; ++i) {
+          float mi, li, x[8];
+          ld_cluster_v2(map_to_rank(ml + 8u * (uint32_t)r, (uint32_t)i), mi, li);
+          if (li == 0.f) continue;                                       // no key of that part: its O may not even exist
+          const float w = ex2_approx(mi - m);
+          const uint32_t base = map_to_rank(part_o + (uint32_t)r * (D * 4u), (uint32_t)i);
+          ld_cluster_v4(base + (uint32_t)((2 * ch) ^ (r & 7)) * 16u, x[0], x[1], x[2], x[3]);
+          ld_cluster_v4(base + (uint32_t)((2 * ch + 1) ^ (r & 7)) * 16u, x[4], x[5], x[6], x[7]);
+          sum = fmaf(w, li, sum);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[e] = fmaf(w, x[e], acc[e]);
+        }
+        const bool live = sum > 0.f;
+        const float inv = live ? 1.f / sum : 0.f;
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = live ? pack2<BF16>(acc[2 * e] * inv, acc[2 * e + 1] * inv) : 0u;
+        const long long tok = tile_tok0 + (r >> P.gp_shift);
+        const int h = head0 + (r & (P.gp - 1));
+        *reinterpret_cast<uint4*>(o_base + tok * P.o_s0 + h * P.o_s1 + ch * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (P.lse != nullptr && ch == 0) P.lse[tok * p.nhead_q + h] = live ? 0.6931471805599453f * (m + log2f(sum)) : -INFINITY;
+      }
+      return true;
+    };
     while (ok) {
       ok = warp_wait(bar_of(bar_item_full, I), par_of(I), abort_flag, budget);
       if (!ok) break;
       const int n_tiles = slots[I & 1].n_tiles;
       if (n_tiles < 0) break;
       const int tile_tok0 = slots[I & 1].tile_tok0, head0 = slots[I & 1].head0, q_end = slots[I & 1].q_end;
-      if (n_tiles == 0) {
+      if (SPLIT ? slots[I & 1].item_tiles <= 0 : n_tiles == 0) {
         // No active k-block: the rows are exact zeros (fwd_triton_fix_tile_size.py:189).
         const int r_tok = tile_tok0 + (row >> P.gp_shift);
-        if (r_tok < q_end) {
+        if (r_tok < q_end && part == 0) {
           uint4* dst = reinterpret_cast<uint4*>(o_base + r_tok * P.o_s0 + (head0 + (row & (P.gp - 1))) * P.o_s1);
 #pragma unroll
           for (int i = 0; i < D / 8; ++i)
@@ -720,6 +803,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
         if (!ok) break;
 
+        if (SPLIT) {
+          ok = finish_part(tile_tok0, head0, q_end, m_ref, l, n_tiles > 0 ? T - 1 : -1);
+          break;                                                         // the CTA's only item; teardown follows
+        }
         // ---- epilogue: O / l -> global; rows past the q-block end are dropped, rows that saw no key are zeros
         if (TRACE && tid == 0) stamp(P.trace, T - 1, 13);
         const bool live = l > 0.f;
@@ -801,7 +888,8 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   // ---- teardown: every thread gets here (all waits are bounded)
   tc_fence_before();
-  __syncthreads();
+  if (SPLIT) cluster_sync();                           // nobody leaves while a peer may read its shared memory
+  else __syncthreads();
   if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TmemCols<D>::value);
@@ -933,7 +1021,14 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   // two persistent CTAs per SM; one above 128 head dimensions (O alone takes 256 of the SM's 512 TMEM columns, the
   // tiles 192 KB of its shared memory)
   const long long resident = (p.headdim > 128 ? 1ll : 2ll) * sm100_sm_count();
-  const unsigned grid = (unsigned)(P.total_items < resident ? P.total_items : resident);
+  // Too few items for the chip: 2, 4 or 8 CTAs share an item, as long as they are needed to fill it and each of them gets 24
+  // tiles of the average sample (the mask, of which the host knows nothing, leaves perhaps a tenth to a third of
+  // them).  Below that the cluster's meeting costs as much as the tiles saved (samples of 16 to 500 keys in parts of 2: 54 -> 64 us).
+  P.split = 1;
+  while (P.split < 8 && P.total_items * P.split < resident && a.total_k / kTileRows / p.batch >= kSplitTiles * 2 * P.split) P.split *= 2;
+  const bool split = P.split > 1 && P.trace == nullptr;
+  if (!split) P.split = 1;
+  const unsigned grid = split ? (unsigned)(P.total_items * P.split) : (unsigned)(P.total_items < resident ? P.total_items : resident);
 
   CUtensorMap tq, tk, tv;
   if (!sm100_encode_map(fn, &tq, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], gp, P.tt) ||
@@ -947,30 +1042,37 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   // innermost extent, the hardware fills those columns of Q, K and V with zeros (so S is exact and the surplus
   // columns of O are zeros), and the epilogue stores the real columns only.
   const int d_tile = p.headdim <= 64 ? 64 : p.headdim <= 128 ? 128 : 256;
-  const size_t smem = (128u + 4u * (size_t)kTileRows) * (size_t)d_tile * 2u + sizeof(Control) + 1024u;
+  size_t smem = (128u + 4u * (size_t)kTileRows) * (size_t)d_tile * 2u + sizeof(Control) + 1024u;
+  // A third CTA on an SM would wait for tensor memory that its neighbours hold while they wait for their clusters: never let one in.
+  if (split && smem < kSplitSmem) smem = kSplitSmem;
   cudaError_t e = cudaSuccess;
   // Programmatic launch (2-3 us less between the two kernels of a forward): the CTAs set up barriers and tensor memory while the schedule kernel is still running.
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)P.split;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-#define HBSA_LAUNCH_SM100(D_, BF_, TR_, GA_)                                                              \
+  cfg.attrs = attr;
+  cfg.numAttrs = split ? 2 : 1;
+#define HBSA_LAUNCH_SM100(D_, BF_, TR_, GA_, SP_)                                                              \
   do {                                                                                                   \
     static SmemOptIn opt_in;                                                                             \
-    e = opt_in.once(reinterpret_cast<const void*>(fwd_sm100_kernel<D_, BF_, TR_, GA_>), (int)smem);       \
-    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fwd_sm100_kernel<D_, BF_, TR_, GA_>, tq, tk, tv, P); \
+    e = opt_in.once(reinterpret_cast<const void*>(fwd_sm100_kernel<D_, BF_, TR_, GA_, SP_>), (int)smem);       \
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fwd_sm100_kernel<D_, BF_, TR_, GA_, SP_>, tq, tk, tv, P); \
   } while (0)
 #define HBSA_LAUNCH_SM100_T(D_, BF_)                                                                      \
   do {                                                                                                   \
-    if (gather) HBSA_LAUNCH_SM100(D_, BF_, false, true);                                                 \
-    else if (P.trace != nullptr) HBSA_LAUNCH_SM100(D_, BF_, true, false);                                \
-    else HBSA_LAUNCH_SM100(D_, BF_, false, false);                                                       \
+    if (split && gather) HBSA_LAUNCH_SM100(D_, BF_, false, true, true);                                   \
+    else if (split) HBSA_LAUNCH_SM100(D_, BF_, false, false, true);                                       \
+    else if (gather) HBSA_LAUNCH_SM100(D_, BF_, false, true, false);                                     \
+    else if (P.trace != nullptr) HBSA_LAUNCH_SM100(D_, BF_, true, false, false);                         \
+    else HBSA_LAUNCH_SM100(D_, BF_, false, false, false);                                                \
   } while (0)
   if (d_tile == 256) { if (bf16) HBSA_LAUNCH_SM100_T(256, true); else HBSA_LAUNCH_SM100_T(256, false); }
   else if (d_tile == 128) { if (bf16) HBSA_LAUNCH_SM100_T(128, true); else HBSA_LAUNCH_SM100_T(128, false); }
