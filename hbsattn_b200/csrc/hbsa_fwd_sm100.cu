@@ -43,8 +43,9 @@
 // mbarriers.  T counts K/V tiles over the whole life of the CTA, I counts published items, Iq those
 // of them that have tiles.  Two-entry barrier arrays are indexed by the low bit of the count and
 // complete once per use, so a waiter for count c uses entry c & 1 and parity (c >> 1) & 1:
-//   k_full / v_full [T]: TMA bytes landed          s_full [T]: S = Q K^T done (K stage free again)
-//   pv_done [T]: O += P V done (V stage free again)
+//   k_full / v_full [T]: TMA bytes landed (entry T modulo the stages)
+//   s_full [T]: S = Q K^T done (K stage free again)    pv_done [T]: O += P V done (V stage free again); rings of more than two
+//   stages have barriers of their own for that (k_free, v_free), since a two-entry barrier cannot be asked about tile T - 4
 // P(T) is handed over through a plain shared-memory counter instead (p_count, one increment per softmax warp, never
 // reset): the issuing thread reads it with an ordinary load in its polling loop.
 //   q_full [Iq]: Q tile landed                     o_free [Iq]: epilogue has read O out of TMEM
@@ -69,6 +70,11 @@ constexpr int kUnitRows = kFwdUnitRows;   // rows of the pieces a gathered tile 
 constexpr int kTileUnits = kTileRows / kUnitRows;
 constexpr int kSplitTiles = 24;           // tiles of a dense row that a CTA of a cluster gets at least
 constexpr size_t kSplitSmem = 80u * 1024u;   // more than a third of an SM's shared memory
+// K and V stages of a CTA.  Two fill its shared memory at 128 head dimensions and more; at 64 four fit.  With two, a tile is requested
+// when the last but one has been multiplied, about one memory latency before it is due: loads were on the critical path wherever K
+// and V come from HBM rather than L2.
+template <int D> struct Stages { static constexpr int value = D == 64 ? 4 : 2; };
+constexpr int kMaxStages = 4;
 constexpr int kNoKey = 0x40000000;        // "first key" of the empty pieces at the end of a row's last gathered tile
 // S0, S1 of 64 columns + O of D columns, rounded up to a power of two
 template <int D> struct TmemCols { static constexpr uint32_t value = D > 128 ? 512u : 256u; };
@@ -123,13 +129,16 @@ struct ItemSlot {
 
 struct __align__(16) Control {
   unsigned long long item_full[2], item_done[2];
-  unsigned long long q_full[2], k_full[2], v_full[2], s_full[2], pv_done[2], o_free[2];
+  unsigned long long q_full[2], k_full[kMaxStages], v_full[kMaxStages], s_full[2], pv_done[2], o_free[2];
+  unsigned long long k_free[kMaxStages], v_free[kMaxStages];    // rings of more than two stages only
   unsigned long long drain;
   unsigned long long parts_ready;   // SPLIT: the partial results of every CTA of the cluster are in shared memory
   uint32_t tmem_base;
   int abort_flag;
   unsigned p_count[2];       // arrivals of the softmax warps for the S buffer tile & 1 (never reset: 4 per tile)
-  __align__(16) int tile_keys[4][kTileUnits];   // in-sample key of the tile's first row (gathered tiles: of every piece)
+  // In-sample key of the tile's first row (gathered tiles: of every piece).  The loader writes entry T once S(T - stages) is done, by
+  // which time the softmax warps have left tile T - stages - 2: twice the stages are enough.
+  __align__(16) int tile_keys[2 * kMaxStages][kTileUnits];
   ItemSlot slot[2];
   float2 part_ml[128];       // SPLIT: reference maximum and row sum of this CTA's part
 };
@@ -173,20 +182,24 @@ __device__ __forceinline__ void exp16(const uint32_t* r, uint32_t (&pk)[8], floa
   ptx::unpack_f32x2(sb, sum[1], sum[3]);
 }
 
+// Barrier entry and parity for the c-th use of a ring of ST (a power of two) stages.
+template <int ST> __device__ __forceinline__ uint32_t ring_bar(uint32_t base, int c) { return base + 8u * (uint32_t)(c & (ST - 1)); }
+template <int ST> __device__ __forceinline__ uint32_t ring_par(int c) { return ((uint32_t)c / ST) & 1u; }
+
 // The issue sequences of the MMA thread.  Every descriptor and TMEM address is precomputed into
 // registers once per CTA, so a product is nothing but back-to-back tcgen05.mma instructions.
 template <int KSTEPS>
-__device__ __forceinline__ void issue_qk(uint32_t tS, const uint64_t (&qd)[KSTEPS], const uint64_t (&kd)[KSTEPS], uint32_t idesc) {
-  ptx::mma_ss_c<false>(tS, qd[0], kd[0], idesc);
+__device__ __forceinline__ void issue_qk(uint32_t tS, const uint64_t (&qd)[KSTEPS], const uint64_t (&kd)[KSTEPS], uint32_t stage_off, uint32_t idesc) {
+  ptx::mma_ss_c<false>(tS, qd[0], kd[0] + stage_off, idesc);
 #pragma unroll
-  for (int ks = 1; ks < KSTEPS; ++ks) ptx::mma_ss_c<true>(tS, qd[ks], kd[ks], idesc);
+  for (int ks = 1; ks < KSTEPS; ++ks) ptx::mma_ss_c<true>(tS, qd[ks], kd[ks] + stage_off, idesc);
 }
 // O (+)= P V of one tile; the first product of an item overwrites O.
-__device__ __forceinline__ void issue_pv(uint32_t tO, const uint32_t (&pa)[4], const uint64_t (&vd)[4], uint32_t idesc, bool first) {
-  if (first) ptx::mma_ts_c<false>(tO, pa[0], vd[0], idesc);
-  else ptx::mma_ts_c<true>(tO, pa[0], vd[0], idesc);
+__device__ __forceinline__ void issue_pv(uint32_t tO, const uint32_t (&pa)[4], const uint64_t (&vd)[4], uint32_t stage_off, uint32_t idesc, bool first) {
+  if (first) ptx::mma_ts_c<false>(tO, pa[0], vd[0] + stage_off, idesc);
+  else ptx::mma_ts_c<true>(tO, pa[0], vd[0] + stage_off, idesc);
 #pragma unroll
-  for (int ks = 1; ks < 4; ++ks) ptx::mma_ts_c<true>(tO, pa[ks], vd[ks], idesc);
+  for (int ks = 1; ks < 4; ++ks) ptx::mma_ts_c<true>(tO, pa[ks], vd[ks] + stage_off, idesc);
 }
 
 // TRACE = true is the instantiation that runs while a debug trace buffer is set; the shipped path carries
@@ -212,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const Sm100Params P) {
   using namespace ptx;
-  constexpr int PANELS = D / 64;
+  constexpr int PANELS = D / 64, ST = Stages<D>::value;
   constexpr uint32_t Q_BYTES = 128u * D * 2u;
   constexpr uint32_t KV_BYTES = (uint32_t)kTileRows * D * 2u;
   const Problem& p = P.p;
@@ -236,12 +249,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const uint32_t pad = ((raw_addr + 1023u) & ~1023u) - raw_addr;
   uint8_t* const smem = smem_raw + pad;
   const uint32_t sQ = raw_addr + pad;
-  const uint32_t sK = sQ + Q_BYTES;                   // 2 stages
-  const uint32_t sV = sK + 2 * KV_BYTES;          // 2 stages
-  Control* const ctl = reinterpret_cast<Control*>(smem + Q_BYTES + 4 * KV_BYTES);
+  const uint32_t sK = sQ + Q_BYTES;
+  const uint32_t sV = sK + ST * KV_BYTES;
+  Control* const ctl = reinterpret_cast<Control*>(smem + Q_BYTES + 2 * ST * KV_BYTES);
   const uint32_t bar_item_full = smem_u32(&ctl->item_full[0]), bar_item_done = smem_u32(&ctl->item_done[0]);
   const uint32_t bar_q_full = smem_u32(&ctl->q_full[0]), bar_k_full = smem_u32(&ctl->k_full[0]);
   const uint32_t bar_v_full = smem_u32(&ctl->v_full[0]), bar_s_full = smem_u32(&ctl->s_full[0]);
+  const uint32_t bar_k_free = smem_u32(&ctl->k_free[0]), bar_v_free = smem_u32(&ctl->v_free[0]);
   const uint32_t bar_pv_done = smem_u32(&ctl->pv_done[0]);
   const uint32_t bar_o_free = smem_u32(&ctl->o_free[0]);
   volatile int* const abort_flag = &ctl->abort_flag;
@@ -252,11 +266,15 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       mbar_init(bar_item_full + 8 * i, 1);
       mbar_init(bar_item_done + 8 * i, kSoftmaxWarps + 1);      // softmax warps + the MMA thread
       mbar_init(bar_q_full + 8 * i, 1);
-      mbar_init(bar_k_full + 8 * i, 1);
-      mbar_init(bar_v_full + 8 * i, 1);
       mbar_init(bar_s_full + 8 * i, 1);
       mbar_init(bar_pv_done + 8 * i, 1);
       mbar_init(bar_o_free + 8 * i, kSoftmaxWarps);
+    }
+    for (int i = 0; i < ST; ++i) {
+      mbar_init(bar_k_full + 8 * i, 1);
+      mbar_init(bar_v_full + 8 * i, 1);
+      mbar_init(bar_k_free + 8 * i, 1);
+      mbar_init(bar_v_free + 8 * i, 1);
     }
     mbar_init(smem_u32(&ctl->drain), 1);
     if (SPLIT) mbar_init(smem_u32(&ctl->parts_ready), (uint32_t)(kSoftmaxWarps * P.split));
@@ -298,40 +316,45 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (SPLIT) next_idx = blockIdx.x / (unsigned)parts;
     else if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
     next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
-    // K and V of tile T into stage T & 1; `key`: the tile's first key (gathered: lane u's is that of piece u)
+    // K and V of tile T into stage T % ST; `key`: the tile's first key (gathered: lane u's is that of piece u)
     auto load_tile = [&](const ItemRecord& rec, int key) {
-      if (T >= 2) ok = warp_wait(bar_of(bar_s_full, T), par_of(T - 2), abort_flag, budget);
+      // K stage T % ST is free once S of tile T - ST is done
+      if (T >= ST) ok = ST == 2 ? warp_wait(bar_of(bar_s_full, T), par_of(T - 2), abort_flag, budget)
+                                : warp_wait(ring_bar<ST>(bar_k_free, T), ring_par<ST>(T - ST), abort_flag, budget);
       if (!ok) return;
+      const uint32_t k_full = ring_bar<ST>(bar_k_full, T), v_full = ring_bar<ST>(bar_v_full, T);
+      const uint32_t dst_k = sK + (uint32_t)(T & (ST - 1)) * KV_BYTES, dst_v = sV + (uint32_t)(T & (ST - 1)) * KV_BYTES;
       // where this lane's box starts: its piece (pieces without keys read past the tensor, which TMA fills with zeros) and panel
       const int unit = lane % kTileUnits, panel = lane / kTileUnits;
       const int unit_key = GATHER ? __shfl_sync(0xffffffffu, key, unit) : 0;
       const int unit_row = unit_key == kNoKey ? P.total_k : rec.k_begin + unit_key;
-      if (GATHER ? lane < kTileUnits : lane == 0) *(volatile int*)&ctl->tile_keys[T & 3][lane] = key;
+      if (GATHER ? lane < kTileUnits : lane == 0) *(volatile int*)&ctl->tile_keys[T & (2 * kMaxStages - 1)][lane] = key;
       __threadfence_block();
       if (GATHER) __syncwarp();
-      if (lane == 0) mbar_arrive_expect_tx(bar_of(bar_k_full, T), KV_BYTES);
+      if (lane == 0) mbar_arrive_expect_tx(k_full, KV_BYTES);
       if (GATHER) {
         __syncwarp();
         if (panel < PANELS)
-          tma_load_3d(sK + (T & 1) * KV_BYTES + panel * KV_PANEL + unit * (kUnitRows * 128u), &tm_k, bar_of(bar_k_full, T), panel * 64, rec.hk, unit_row);
+          tma_load_3d(dst_k + panel * KV_PANEL + unit * (kUnitRows * 128u), &tm_k, k_full, panel * 64, rec.hk, unit_row);
       } else if (lane == 0) {
 #pragma unroll
         for (int pn = 0; pn < PANELS; ++pn)
-          tma_load_3d(sK + (T & 1) * KV_BYTES + pn * KV_PANEL, &tm_k, bar_of(bar_k_full, T), pn * 64, rec.hk, rec.k_begin + key);
+          tma_load_3d(dst_k + pn * KV_PANEL, &tm_k, k_full, pn * 64, rec.hk, rec.k_begin + key);
       }
       if (TRACE && lane == 0) stamp(P.trace, T, 0);
-      // V stage T & 1 is free once the P V product of tile T-2 is done
-      if (T >= 2) ok = warp_wait(bar_of(bar_pv_done, T), par_of(T - 2), abort_flag, budget);
+      // V stage T % ST is free once the P V product of tile T - ST is done
+      if (T >= ST) ok = ST == 2 ? warp_wait(bar_of(bar_pv_done, T), par_of(T - 2), abort_flag, budget)
+                                : warp_wait(ring_bar<ST>(bar_v_free, T), ring_par<ST>(T - ST), abort_flag, budget);
       if (!ok) return;
-      if (lane == 0) mbar_arrive_expect_tx(bar_of(bar_v_full, T), KV_BYTES);
+      if (lane == 0) mbar_arrive_expect_tx(v_full, KV_BYTES);
       if (GATHER) {
         __syncwarp();
         if (panel < PANELS)
-          tma_load_3d(sV + (T & 1) * KV_BYTES + panel * KV_PANEL + unit * (kUnitRows * 128u), &tm_v, bar_of(bar_v_full, T), panel * 64, rec.hk, unit_row);
+          tma_load_3d(dst_v + panel * KV_PANEL + unit * (kUnitRows * 128u), &tm_v, v_full, panel * 64, rec.hk, unit_row);
       } else if (lane == 0) {
 #pragma unroll
         for (int pn = 0; pn < PANELS; ++pn)
-          tma_load_3d(sV + (T & 1) * KV_BYTES + pn * KV_PANEL, &tm_v, bar_of(bar_v_full, T), pn * 64, rec.hk, rec.k_begin + key);
+          tma_load_3d(dst_v + pn * KV_PANEL, &tm_v, v_full, pn * 64, rec.hk, rec.k_begin + key);
       }
       if (TRACE && lane == 0) stamp(P.trace, T, 1);
       ++T;
@@ -375,8 +398,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (n_tiles <= 0) continue;
 
       // Q has one buffer: the previous item's last S (tile T-1) must be done.  S products complete in
-      // order, so this covers tile T-2 (whose K stage the first tile of this item reuses) as well.
-      if (T >= 1) ok = warp_wait(bar_of(bar_s_full, T - 1), par_of(T - 1), abort_flag, budget);
+      // order, so this covers all earlier tiles as well.  (In a ring of four the loader may be two uses of an s_full entry
+      // ahead of the products, where that entry's parity would read as done.)
+      if (T >= 1) ok = ST == 2 ? warp_wait(bar_of(bar_s_full, T - 1), par_of(T - 1), abort_flag, budget)
+                               : warp_wait(ring_bar<ST>(bar_k_free, T - 1), ring_par<ST>(T - 1), abort_flag, budget);
       if (!ok) break;
       if (lane == 0) {
         mbar_arrive_expect_tx(bar_of(bar_q_full, Iq), Q_BYTES);
@@ -440,9 +465,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     if (!ok) {
       // Gave up: let the copies already issued land before the CTA retires (bounded).
-      for (int back = 1; back <= 2 && T - back >= 0; ++back) {
-        mbar_wait_bounded(bar_of(bar_k_full, T - back), par_of(T - back), abort_flag, budget >> 4);
-        mbar_wait_bounded(bar_of(bar_v_full, T - back), par_of(T - back), abort_flag, budget >> 4);
+      for (int back = 1; back <= ST && T - back >= 0; ++back) {
+        mbar_wait_bounded(ring_bar<ST>(bar_k_full, T - back), ring_par<ST>(T - back), abort_flag, budget >> 4);
+        mbar_wait_bounded(ring_bar<ST>(bar_v_full, T - back), ring_par<ST>(T - back), abort_flag, budget >> 4);
       }
     }
   } else if (warp == kMmaWarp) {
@@ -507,7 +532,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (pT < qT) {
           // one probe per idle turn in the steady state: that V(pT) has landed is looked up once and remembered
           if (!v_landed) {
-            v_landed = mbar_test(bar_of(bar_v_full, pT), par_of(pT));
+            v_landed = mbar_test(ring_bar<ST>(bar_v_full, pT), ring_par<ST>(pT));
             if (TRACE && v_landed) stamp(P.trace, pT, 18);
           }
           const bool p_there = *(volatile unsigned*)&ctl->p_count[pT & 1] >= (unsigned)kSoftmaxWarps * ((unsigned)(pT >> 1) + 1u);
@@ -527,8 +552,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             tc_fence_after();
 #endif
             if (TRACE) stamp(P.trace, pT, 4);
-            if (pT & 1) issue_pv(tO, pa1, vd1, idesc_pv, (fl & 1) != 0);
-            else issue_pv(tO, pa0, vd0, idesc_pv, (fl & 1) != 0);
+            // descriptors of stage 0 or 1, and 0 or 2 stages (in 16-byte units) further in a ring of four
+            const uint32_t off = ST > 2 ? (uint32_t)(pT & (ST - 2)) * (KV_BYTES >> 4) : 0u;
+            if (pT & 1) issue_pv(tO, pa1, vd1, off, idesc_pv, (fl & 1) != 0);
+            else issue_pv(tO, pa0, vd0, off, idesc_pv, (fl & 1) != 0);
+            if (ST > 2) tc_commit(ring_bar<ST>(bar_v_free, pT));
             tc_commit(bar_of(bar_pv_done, pT));
             if (TRACE) stamp(P.trace, pT, 5);
             if (fl & 1) ++pIq;
@@ -540,7 +568,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           }
         }
         if (q_have && qT < pT + 2) {
-          bool ready = mbar_test(bar_of(bar_k_full, qT), par_of(qT));
+          bool ready = mbar_test(ring_bar<ST>(bar_k_full, qT), ring_par<ST>(qT));
           if (ready && q_first) ready = mbar_test(bar_of(bar_q_full, qIq), par_of(qIq));
 #ifdef HBSA_STRICT_TCGEN05
           // S(t) overwrites the columns of P(t-2): wait until P V(t-2) has completed instead of relying on the
@@ -551,9 +579,11 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           if (ready) {
             if (TRACE) stamp(P.trace, qT, 2);
             const uint32_t tSb = tmem_base + (uint32_t)(qT & 1) * kSStride;
-            if (qT & 1) issue_qk<D / 16>(tSb, qd, kd1, idesc_qk);
-            else issue_qk<D / 16>(tSb, qd, kd0, idesc_qk);
+            const uint32_t off = ST > 2 ? (uint32_t)(qT & (ST - 2)) * (KV_BYTES >> 4) : 0u;
+            if (qT & 1) issue_qk<D / 16>(tSb, qd, kd1, off, idesc_qk);
+            else issue_qk<D / 16>(tSb, qd, kd0, off, idesc_qk);
             tc_commit(bar_of(bar_s_full, qT));
+            if (ST > 2) tc_commit(ring_bar<ST>(bar_k_free, qT));
             if (TRACE) stamp(P.trace, qT, 3);
             const int fl_new = (q_first ? 1 : 0) | (q_left == 1 ? 2 : 0) | (qI << 2);
             if (qT & 1) fl1 = fl_new; else fl0 = fl_new;
@@ -682,9 +712,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             col_limit = -1;
 #pragma unroll
             for (int u = 0; u < kTileUnits; ++u)
-              col_limit += min(max(limit_row + 1 - *(volatile int*)&ctl->tile_keys[T & 3][u], 0), kUnitRows);
+              col_limit += min(max(limit_row + 1 - *(volatile int*)&ctl->tile_keys[T & (2 * kMaxStages - 1)][u], 0), kUnitRows);
           } else {
-            col_limit = limit_row - *(volatile int*)&ctl->tile_keys[T & 3][0];
+            col_limit = limit_row - *(volatile int*)&ctl->tile_keys[T & (2 * kMaxStages - 1)][0];
           }
           const uint32_t tSmine = tmem_base + (uint32_t)(T & 1) * kSStride + lane_off;
 
@@ -1042,7 +1072,7 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   // innermost extent, the hardware fills those columns of Q, K and V with zeros (so S is exact and the surplus
   // columns of O are zeros), and the epilogue stores the real columns only.
   const int d_tile = p.headdim <= 64 ? 64 : p.headdim <= 128 ? 128 : 256;
-  size_t smem = (128u + 4u * (size_t)kTileRows) * (size_t)d_tile * 2u + sizeof(Control) + 1024u;
+  size_t smem = (128u + 2u * (d_tile == 64 ? Stages<64>::value : Stages<128>::value) * (size_t)kTileRows) * (size_t)d_tile * 2u + sizeof(Control) + 1024u;
   // A third CTA on an SM would wait for tensor memory that its neighbours hold while they wait for their clusters: never let one in.
   if (split && smem < kSplitSmem) smem = kSplitSmem;
   cudaError_t e = cudaSuccess;
