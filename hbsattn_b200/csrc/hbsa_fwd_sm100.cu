@@ -704,7 +704,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // Rows of an M tile that exist come first.  A warp without any (decoding, q-blocks of fewer than 128 rows, ragged ends)
         // leaves S as it is, since a row of P V depends on its own row of P only and the epilogue drops it.  It still answers for
         // every tile, in order, so that the count of a tile stays four.  Same GPU, same bits: one new token on 16 long contexts
-        // 89.8 -> 72.5 us, 80x48 blocks with 4 heads a group 7.97 -> 6.91 ms, blocks of 64 rows 228 -> 196 us.
+        // 89.8 -> 72.5 us, blocks of 64 rows at d = 96 228 -> 196 us.
         const bool idle_warp = tile_tok0 + ((warp * 32) >> P.gp_shift) >= q_end;
         if (TRACE && tid == 0) stamp(P.trace, T, 10);
         for (int t = 0; t < n_tiles && ok; ++t, ++T) {
