@@ -87,6 +87,7 @@ struct __align__(16) BwdControl {
   unsigned long long strm_full[kBwdStages], strm_free[kBwdStages];
   unsigned long long s_full[2], dp_full[2], p_ready[2], ds_ready[2];
   unsigned long long acc_full, acc_free, drain;
+  unsigned long long ragged_full;             // the copies of a tile with rows to clear (see zero_rows)
   uint32_t tmem_base;
   int abort_flag;
   int info0[kBwdStages], info1[kBwdStages];   // KV: key limit of the tile's first token; dQ: first key, one past the last key
@@ -117,6 +118,22 @@ __device__ __forceinline__ float fp16_grad_factor(const BwdHeader* h, int headdi
   if (!(bound > 0.f) || !isfinite(bound)) return 1.f;
   const int e = 13 - ilogbf(bound);
   return ldexpf(1.f, e < -60 ? -60 : e > 60 ? 60 : e);
+}
+
+// Streamed rows that take part in no pair: past the end of the q-block or k-block (they hold whatever follows in the packed
+// tensor: the next block or sample, or memory behind the last one) and rows of q that see no key.  Masking gives them a P of zero, but
+// 0 x NaN and 0 x Inf would still come out of dP and of the accumulating products.  So the loader clears them once the tile has
+// landed and hands the tile over afterwards; every use of them is then 0 x 0.  A row is 128 bytes per 64-dim panel, whatever the swizzle.
+// Isolation is by block: elements that a causal mask cuts out of an active pair are multiplied by an exact zero.
+// (Clearing by the elementwise warps between the first and second products, with selects on S and dP, made the hot loop 6 % slower.)
+template <int D>
+__device__ __forceinline__ void zero_rows(uint32_t tile, uint32_t y_off, uint32_t panel_bytes, unsigned long long gone, int lane) {
+  constexpr int CHUNKS = D / 8;                  // 16-byte pieces of a row
+  const int piece = lane % CHUNKS, which = lane / CHUNKS;
+  const uint32_t base = tile + (which ? y_off : 0u) + (uint32_t)(piece >> 3) * panel_bytes + (uint32_t)(piece & 7) * 16u;
+  for (; gone != 0ull; gone &= gone - 1ull)
+    if (which < 2) ptx::st_shared_v4(base + (uint32_t)(__ffsll((long long)gone) - 1) * 128u, 0u, 0u, 0u, 0u);
+  ptx::fence_proxy_async();
 }
 
 // acc (+)= A[tmem] B over `n` 16-wide k-steps.
@@ -184,6 +201,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     mbar_init(b_acc_full, 1);
     mbar_init(b_acc_free, kBwdEwWarps);
     mbar_init(smem_u32(&ctl->drain), 1);
+    mbar_init(smem_u32(&ctl->ragged_full), 1);
     // the tiles need a 1024-byte aligned base; without static shared memory the dynamic part has one
     ctl->abort_flag = (sStat & 1023u) != 0 ? 1 : 0;
     fence_barrier_init();
@@ -210,6 +228,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     unsigned long long* const cursor = &P.head->cursor[KV ? 1 : 0];
     int I = 0, Iq = 0, T = 0, stage = 0;
     uint32_t stage_par = 1u;                       // parity of "stage free" for the current round (first round: free)
+    uint32_t ragged_par = 0u;                      // parity of the next tile with rows to clear
     bool ok = *abort_flag == 0;
     long long next_idx = 0;
     if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
@@ -242,7 +261,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       ++Iq;
     };
-    // one streamed tile; KV: `valid` tokens of it are real, their {-lse, delta} pairs go along
+    // one streamed tile; its first `valid` tokens (KV) or keys (dQ) are the block's.  KV: the {-lse, delta} pairs of the rows go along
     auto load_tile = [&](int row0, int head0, int valid, int i0, int i1) {
       float2 st0 = make_float2(-INFINITY, 0.f), st1 = st0;
       if (KV) {
@@ -258,18 +277,38 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         ctl->delta[stage][lane] = st0.y;
         ctl->delta[stage][lane + 32] = st1.y;
       }
+      unsigned long long gone;                       // rows to clear
+      if (KV) {
+        const uint32_t g0 = __ballot_sync(0xffffffffu, lane < nt && st0.x == -INFINITY);
+        const uint32_t g1 = __ballot_sync(0xffffffffu, lane + 32 < nt && st1.x == -INFINITY);
+        gone = (unsigned long long)g1 << 32 | g0;
+      } else {
+        gone = valid < nt ? ((nt < 64 ? 1ull << nt : 0ull) - 1ull) & ~((1ull << valid) - 1ull) : 0ull;
+      }
+      const uint32_t dst = sStrm + (uint32_t)stage * 2u * STRM;
       __syncwarp();
       if (lane == 0) {
         ctl->info0[stage] = i0;
         ctl->info1[stage] = i1;
         __threadfence_block();
-        const uint32_t bar = b_strm_full + 8u * stage, dst = sStrm + (uint32_t)stage * 2u * STRM;
+        const uint32_t bar = gone != 0ull ? smem_u32(&ctl->ragged_full) : b_strm_full + 8u * stage;
         mbar_arrive_expect_tx(bar, 2u * (uint32_t)nt * D * 2u);
 #pragma unroll
         for (int pn = 0; pn < PANELS; ++pn) {
           tma_load_3d(dst + pn * strm_panel, &tm_x, bar, pn * 64, head0, row0);
           tma_load_3d(dst + STRM + pn * strm_panel, &tm_y, bar, pn * 64, head0, row0);
         }
+      }
+      if (gone != 0ull) {
+        ok = warp_wait(smem_u32(&ctl->ragged_full), ragged_par, abort_flag, budget);
+        if (!ok) {                                   // the copy is still in flight: bounded, like the others at the end
+          mbar_wait_clock(smem_u32(&ctl->ragged_full), ragged_par, budget >> 4);
+          return;
+        }
+        ragged_par ^= 1u;
+        zero_rows<D>(dst, STRM, strm_panel, gone, lane);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(b_strm_full + 8u * stage);
       }
       ++T;
       if (++stage == kBwdStages) {
@@ -376,8 +415,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const int pos = __ffs(bal) - 1;
             bal &= bal - 1;
             const int blk0 = __shfl_sync(0xffffffffu, val, pos) * p.kbs;
-            const int k_end = min(blk0 + p.kbs, rec.k_stop);
-            for (int k0 = blk0; k0 < k_end && ok; k0 += nt) load_tile(rec.k_begin + k0, rec.hk, nt, k0, k_end);
+            const int blk_end = min(blk0 + p.kbs, rec.k_len), k_end = min(blk_end, rec.k_stop);
+            for (int k0 = blk0; k0 < k_end && ok; k0 += nt) load_tile(rec.k_begin + k0, rec.hk, blk_end - k0, k0, k_end);
           }
         }
       }
@@ -517,12 +556,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       const int hq = KV ? 0 : head + (row & (P.gp - 1));
       const int key = pos0 + row;
       float neg_lse = -INFINITY, delta = 0.f;
+      bool no_keys = false;                        // dQ: the row's log-sum-exp says that it saw no key
       int limit_row = k_len - 1;
       if (!KV) {
         if (valid && n_tiles > 0) {
           const float2 st = P.stats[(long long)tok * p.nhead_q + hq];
           neg_lse = st.x;
           delta = st.y;
+          no_keys = neg_lse == -INFINITY;
         }
         if (p.causal) limit_row = min(limit_row, pos0 + (row >> P.gp_shift) + off);
       }
@@ -662,7 +703,8 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             if (c_base + cb + c < p.headdim) {
               uint32_t w[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) w[e] = pack2<BF16>(__uint_as_float(a[c + 2 * e]) * mul, __uint_as_float(a[c + 2 * e + 1]) * mul);
+              for (int e = 0; e < 4; ++e)
+                w[e] = !KV && no_keys ? 0u : pack2<BF16>(__uint_as_float(a[c + 2 * e]) * mul, __uint_as_float(a[c + 2 * e + 1]) * mul);
               *reinterpret_cast<uint4*>(orow + c_base + cb + c) = make_uint4(w[0], w[1], w[2], w[3]);
             }
           }
@@ -723,7 +765,7 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams P, const uint16
     if (row < rows) {
       if (chunk == 0) {
         const float l = lse[row];
-        stats[row] = l > -INFINITY ? make_float2(-l * kLog2e, acc) : make_float2(-INFINITY, 0.f);
+        stats[row] = fabsf(l) < INFINITY ? make_float2(-l * kLog2e, acc) : make_float2(-INFINITY, 0.f);
       }
       if ((tok < q_lo || tok >= q_hi) && chunk < n_chunk) *reinterpret_cast<uint4*>(dq + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
     }
