@@ -252,7 +252,7 @@ int hbsa_block_decisions(const hbsa_forward_args* args, uint8_t* decisions, int3
 
 static size_t backward_bytes(int64_t total_q, int64_t total_k, int nhead_q, int nhead_k, int headdim) {
   const size_t generic = hbsa::backward_workspace_bytes(total_q, total_k, nhead_q, nhead_k, headdim);
-  const size_t sm100 = hbsa::backward_sm100_workspace_bytes(total_q, nhead_q);
+  const size_t sm100 = hbsa::backward_sm100_workspace_bytes(total_q, total_k, nhead_q, nhead_k);
   return generic > sm100 ? generic : sm100;        // the dtype and the strides that decide between the two are not known here
 }
 

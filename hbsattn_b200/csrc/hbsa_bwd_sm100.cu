@@ -12,11 +12,25 @@
 // Recomputing S and dP in both launches costs two of seven products but leaves every gradient element with exactly one
 // writer: no fp32 accumulators in memory, no atomics, no conversion pass, and bit-identical results from run to run.
 //
-// P and dS enter the second products as the sum of two 16-bit terms (hi + lo, 16 significant bits for bf16, 22 for fp16),
-// so that no precision is lost against an fp32 product; that doubles three of the seven products, which is what
-// bounds the kernel: per 128x64 tile at d = 128 the tensor pipe is occupied 16 x 47 clocks by the two first products (N = 64
-// operands from shared memory) and 32 x 64 (dK/dV) or 16 x 64 (dQ) by the second ones.  fp16 dS is scaled by a power of two
-// taken from max|dO| max|V| d beforehand, so that neither small nor large (loss-scaled) gradients leave its range.
+// P and dS enter the second products as the sum of two 16-bit terms (hi + lo), which doubles three of the seven products and is
+// what bounds the kernel: per 128x64 tile at d = 128 the tensor pipe is occupied 16 x 47 clocks by the two first products (N = 64
+// operands from shared memory) and 32 x 64 (dK/dV) or 16 x 64 (dQ) by the second ones.
+//
+// Precision of the pair.  bf16: 16 significant bits at any magnitude, against the 8 that the gradients are rounded to.  fp16: 22 bits
+// down to 2^-3, and 2^-25 absolutely below (fp16 ends at 2^-24).  So P and dS are scaled by powers of two, of their own for
+// every row of the stationary tile (a key in dK/dV, a row of q in dQ; a row of an accumulator can be scaled back exactly):
+//   first launch   2^15 P;  dS by 2^13 / (|dO row| max|V|) (dQ) or 2^13 / (max|dO| max|V|) (dK/dV), which keeps it below 2^15.
+//                  The largest |P| and |dS| of every row are kept track of on the way.
+//   second launch  items in which a row's largest value stayed below 2^-9 sqrt(tiles) (keys that share their queries with an attention sink,
+//                  rows whose dO is far below their neighbours') or went above 2^16 are done again with powers of two that
+//                  bring every row's largest value to 2^14.  What is lost then is 2^-39 of it: less than the fp32 sums lose.
+// The norms and maxima are those of the sample and kv-head alone: a gradient does not depend on the rest of the batch.
+// Relative error (2-norm) against float64, CUDA-core kernels with fp32 P and dS -> these: 8 ragged samples, d = 64, fp16: dQ 2.1417e-4 ->
+// 2.1410e-4, dK 2.1089e-4 -> 2.1081e-4, dV 2.0751e-4 -> 2.0754e-4; two samples of up to 4096, d = 128, bf16: dQ 1.9083e-3 -> 1.9067e-3,
+// dK 1.8955e-3 -> 1.8944e-3, dV 1.6515e-3 -> 1.6515e-3.  dV of fp16 keys beside a sink (CUDA cores / P unscaled / these): sink 16
+// above, 8192 keys, dO of 256: 2.08e-4 / 0.17 / 2.09e-4; 20 above, 4096 keys, dO of 1024: 2.26e-4 / 1.0 / 2.26e-4.  Nearly flat fp16
+// rows over 16384 keys: 2.21e-4 / 3.50e-4 / 2.25e-4; what is left there comes from the length of the fp32 accumulation (2048 products
+// in a row).  The scales and the redo launch take 2 % of the ragged fp16 training step above.
 //
 // 320 threads, one persistent CTA per SM (TMEM: two tile buffers of 64 S + 64 dP columns, two accumulators of 128):
 //   warps 0-3 / 4-7   elementwise work on the even / odd tiles (thread = TMEM lane), then the epilogue: dV / dK, or the two
@@ -46,18 +60,45 @@ constexpr uint32_t kBwdBuf = 128u;     // TMEM columns of one S + dP buffer
 constexpr uint32_t kBwdAcc = 256u;     // first accumulator column
 constexpr float kLog2e = 1.4426950408889634f;
 
-// First words of the gradient workspace: work cursors of the two launches, running maxima of |dO| and |V| (float bits).
+// First words of the gradient workspace: work cursors of the launches (dQ, dK/dV, and the two that do items again), and the number of
+// items that have to be done again (dQ, dK/dV).
 struct BwdHeader {
-  unsigned long long cursor[2];
-  unsigned int amax_do, amax_v;
+  unsigned long long cursor[4];
+  unsigned long long redo_count[2];
 };
-constexpr size_t kBwdHeaderBytes = 256;
+
+// The gradient workspace; everything from `norm_do` on is used with fp16 only.  A sample's maxima are kept at its first token.
+struct BwdSpace {
+  BwdHeader* head;
+  float2* stats;               // [total_q, nhead_q] {-lse * log2 e (-inf: row without keys), delta}
+  unsigned int* max_do;        // [total_q, nhead_k] largest |dO row| of the sample's rows of the group (bits of a non-negative float)
+  unsigned int* max_v;         // [total_k, nhead_k] largest |V row|
+  float* norm_do;              // [total_q, nhead_q]
+  uint16_t *top_q, *top_k;     // [total_q, nhead_q], [total_k, nhead_k]: biased exponents of the row's largest |P| (low byte, dK/dV) and |dS|
+  long long *redo_q, *redo_k;  // items to do again: each owns at least one row
+};
+// Carves the workspace at `base`; returns its size.  `zeroed`: bytes at the front that start as zeros.
+size_t carve_space(char* base, long long q_tokens, long long k_tokens, int nhead_q, int nhead_k, BwdSpace* s, size_t* zeroed) {
+  char* p = base;
+  auto take = [&](size_t bytes) { char* r = p; p += (bytes + 255) / 256 * 256; return r; };
+  const size_t rows_q = (size_t)q_tokens * nhead_q, rows_k = (size_t)k_tokens * nhead_k;
+  s->head = reinterpret_cast<BwdHeader*>(take(sizeof(BwdHeader)));
+  s->max_do = reinterpret_cast<unsigned int*>(take((size_t)q_tokens * nhead_k * 4));
+  s->max_v = reinterpret_cast<unsigned int*>(take(rows_k * 4));
+  *zeroed = (size_t)(p - base);
+  s->stats = reinterpret_cast<float2*>(take(rows_q * sizeof(float2)));
+  s->norm_do = reinterpret_cast<float*>(take(rows_q * 4));
+  s->top_q = reinterpret_cast<uint16_t*>(take(rows_q * 2));
+  s->top_k = reinterpret_cast<uint16_t*>(take(rows_k * 2));
+  s->redo_q = reinterpret_cast<long long*>(take(rows_q * 8));
+  s->redo_k = reinterpret_cast<long long*>(take(rows_k * 8));
+  return (size_t)(p - base);
+}
 
 struct BwdParams {
   Problem p;
   Workspace ws;
-  BwdHeader* head;
-  const float2* stats;         // [total_q, nhead_q] {-lse * log2 e (-inf: row without keys), delta}
+  BwdSpace sp;
   void *out0, *out1;           // dv, dk (KV) or dq
   int total_q, total_k;
   int gp, gp_shift, n_head_sub;      // q-heads packed into one tile of q rows, tiles of heads per group
@@ -70,6 +111,8 @@ struct BwdParams {
   long long wait_budget;
 };
 
+struct BwdMaps { CUtensorMap a, b, x, y; };      // stationary pair, streamed pair
+
 struct BwdItem {
   int n_tiles;                 // < 0: no more work
   int row0;                    // first stationary row (token) in the packed tensors
@@ -77,19 +120,23 @@ struct BwdItem {
   int head;                    // KV: kv-head; dQ: first q-head
   int pos0;                    // in-sample position of the first stationary row
   int k_len, off;
-  int pad;
+  int first;                   // first token of the sample's queries (KV) or keys (dQ)
+  long long index;             // of the item
 };
 
 struct __align__(16) BwdControl {
   float neg_lse[kBwdStages][kBwdTile];
-  float delta[kBwdStages][kBwdTile];
+  float neg_delta[kBwdStages][kBwdTile];
   unsigned long long item_full[2], item_done[2], stat_full[2], stat_free[2];
   unsigned long long strm_full[kBwdStages], strm_free[kBwdStages];
   unsigned long long s_full[2], dp_full[2], p_ready[2], ds_ready[2];
   unsigned long long acc_full, acc_free, drain;
+  unsigned long long top_ready[2];            // the exponents in `top` are there
   unsigned long long ragged_full;             // the copies of a tile with rows to clear (see zero_rows)
   uint32_t tmem_base;
   int abort_flag;
+  int redo_mark;                              // fp16: 1 + the last item that was put on the redo list
+  uint16_t top[2][128];                       // fp16: exponents of the rows' largest |P| (dQ: keys seen) and |dS| in the tiles of warps 4-7
   int info0[kBwdStages], info1[kBwdStages];   // KV: key limit of the tile's first token; dQ: first key, one past the last key
   BwdItem slot[2];
 };
@@ -109,16 +156,33 @@ template <bool BF16> __device__ __forceinline__ void split2(float x0, float x1, 
   hi = pack2<BF16>(x0, x1);
   float h0, h1;
   unpack16<BF16>(hi, h0, h1);
-  lo = pack2<BF16>(x0 - h0, x1 - h1);
+  float l0, l1;
+  ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(h0, h1), ptx::pack_f32x2(-1.f, -1.f), ptx::pack_f32x2(x0, x1)), l0, l1);
+  lo = pack2<BF16>(l0, l1);
 }
 
-// Power of two that brings |dO V^T| and |delta| below 2^14 (both are bounded by max|dO| max|V| d).
-__device__ __forceinline__ float fp16_grad_factor(const BwdHeader* h, int headdim) {
-  const float bound = __uint_as_float(h->amax_do) * __uint_as_float(h->amax_v) * (float)headdim;
-  if (!(bound > 0.f) || !isfinite(bound)) return 1.f;
-  const int e = 13 - ilogbf(bound);
-  return ldexpf(1.f, e < -60 ? -60 : e > 60 ? 60 : e);
+__device__ __forceinline__ float pow2(int e) { return __int_as_float((max(min(e, 127), -126) + 127) << 23); }
+__device__ __forceinline__ int exponent_of(float x) { return (int)((__float_as_uint(x) >> 23) & 255u); }     // biased; 255: Inf or NaN
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
+
+constexpr int kPShift = 15;          // fp16: P enters its products as 2^15 P
+constexpr int kTopHigh = 127 + 16, kTopGoal = 127 + 14;
+// The smallest exponent of a row's largest value that will do.  Every value of the row is off by at most 2^-25, evenly spread (2^-26.8
+// in the mean), so a sum over n tiles of 64 by 2^-23.8 sqrt(n): 2^-14 or less of the largest value from 2^-9 sqrt(n) on, a quarter
+// of what the rounding of the fp16 result loses, and that only where one value stands alone among very small ones.
+__device__ __forceinline__ int top_low(int n_tiles) { return 127 - 9 + (32 - __clz(n_tiles)) / 2; }
+// fp16: exponent that keeps |dP - delta|, at most 2 * bound, below 2^15
+__device__ __forceinline__ int ds_exponent(float bound) {
+  const int e = exponent_of(bound);
+  return e == 0 || e == 255 ? 0 : max(min(kTopGoal - 1 - e, 100), -100);
+}
+// fp16: a row whose largest value has this exponent is done again (zero, Inf and NaN stay what they are)
+__device__ __forceinline__ bool out_of_range(int top, int low) { return (top > 0 && top < low) || (top >= kTopHigh && top < 255); }
+__device__ __forceinline__ int redo_exponent(int top) { return top > 0 && top < 255 ? kTopGoal - top : 0; }
 
 // Streamed rows that take part in no pair: past the end of the q-block or k-block (they hold whatever follows in the packed
 // tensor: the next block or sample, or memory behind the last one) and rows of q that see no key.  Masking gives them a P of zero, but
@@ -147,10 +211,11 @@ __device__ __forceinline__ void issue_ts(uint32_t acc, uint32_t a_tmem, uint64_t
   }
 }
 
-template <int D, bool BF16, bool KV>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_x,
-                 const __grid_constant__ CUtensorMap tm_y, const BwdParams P) {
+// REDO: the launch that does the items of the redo list again, with the scales that their rows need (fp16).
+// `block` of `blocks`: the CTA's place among those of the launch that do this half.
+template <int D, bool BF16, bool KV, bool REDO>
+__device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_x, const CUtensorMap& tm_y,
+                                         const BwdParams& P, unsigned block, unsigned blocks) {
   // a, b: stationary pair (K, V or Q, dO); x, y: streamed pair (Q, dO or K, V)
   using namespace ptx;
   constexpr int PANELS = D / 64;
@@ -161,9 +226,11 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   OutT* const out1 = static_cast<OutT*>(P.out1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+  const long long total_items = REDO ? (long long)P.sp.head->redo_count[KV ? 1 : 0] : P.total_items;
+  if (REDO && total_items == 0) return;
   if (P.ws.status[0] != HBSA_STATUS_OK) {       // inconsistent block counts: zero gradients
     const long long n = KV ? (long long)P.total_k * p.nhead_k * p.headdim : (long long)P.total_q * p.nhead_q * p.headdim;
-    for (long long i = (long long)blockIdx.x * kBwdThreads + tid; i < n; i += (long long)gridDim.x * kBwdThreads) {
+    for (long long i = (long long)block * kBwdThreads + tid; i < n; i += (long long)blocks * kBwdThreads) {
       out0[i] = OutT(0.f);
       if (KV) out1[i] = OutT(0.f);
     }
@@ -193,6 +260,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       mbar_init(b_dp_full + 8 * i, 1);
       mbar_init(b_p_ready + 8 * i, kBwdEwWarps / 2);
       mbar_init(b_ds_ready + 8 * i, kBwdEwWarps / 2);
+      mbar_init(smem_u32(&ctl->top_ready[i]), kBwdEwWarps / 2);
     }
     for (int i = 0; i < kBwdStages; ++i) {
       mbar_init(b_strm_full + 8 * i, 1);
@@ -203,6 +271,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     mbar_init(smem_u32(&ctl->drain), 1);
     mbar_init(smem_u32(&ctl->ragged_full), 1);
     // the tiles need a 1024-byte aligned base; without static shared memory the dynamic part has one
+    ctl->redo_mark = 0;
     ctl->abort_flag = (sStat & 1023u) != 0 ? 1 : 0;
     fence_barrier_init();
   }
@@ -225,7 +294,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       prefetch_tensormap(&tm_x);
       prefetch_tensormap(&tm_y);
     }
-    unsigned long long* const cursor = &P.head->cursor[KV ? 1 : 0];
+    unsigned long long* const cursor = &P.sp.head->cursor[(KV ? 1 : 0) + (REDO ? 2 : 0)];
     int I = 0, Iq = 0, T = 0, stage = 0;
     uint32_t stage_par = 1u;                       // parity of "stage free" for the current round (first round: free)
     uint32_t ragged_par = 0u;                      // parity of the next tile with rows to clear
@@ -234,13 +303,14 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
     next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
 
-    auto publish = [&](int n_tiles, int row0, int end, int head, int pos0, int k_len, int off) {
+    auto publish = [&](int n_tiles, int row0, int end, int head, int pos0, int k_len, int off, int first, long long index) {
       if (I >= 2) ok = warp_wait(bar_of(b_item_done, I), par_of(I - 2), abort_flag, budget);
       if (!ok) return;
       if (lane == 0) {
         volatile BwdItem* sl = &ctl->slot[I & 1];
         sl->n_tiles = n_tiles; sl->row0 = row0; sl->end = end; sl->head = head;
         sl->pos0 = pos0; sl->k_len = k_len; sl->off = off;
+        sl->first = first; sl->index = index;
         __threadfence_block();
         mbar_arrive(bar_of(b_item_full, I));
       }
@@ -266,16 +336,16 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       float2 st0 = make_float2(-INFINITY, 0.f), st1 = st0;
       if (KV) {
         const int c1 = lane + 32, h = P.gp - 1;
-        if ((lane >> P.gp_shift) < valid && lane < nt) st0 = P.stats[(long long)(row0 + (lane >> P.gp_shift)) * p.nhead_q + head0 + (lane & h)];
-        if ((c1 >> P.gp_shift) < valid && c1 < nt) st1 = P.stats[(long long)(row0 + (c1 >> P.gp_shift)) * p.nhead_q + head0 + (c1 & h)];
+        if ((lane >> P.gp_shift) < valid && lane < nt) st0 = P.sp.stats[(long long)(row0 + (lane >> P.gp_shift)) * p.nhead_q + head0 + (lane & h)];
+        if ((c1 >> P.gp_shift) < valid && c1 < nt) st1 = P.sp.stats[(long long)(row0 + (c1 >> P.gp_shift)) * p.nhead_q + head0 + (c1 & h)];
       }
       if (T >= kBwdStages) ok = warp_wait(b_strm_free + 8u * stage, stage_par, abort_flag, budget);
       if (!ok) return;
       if (KV) {
-        ctl->neg_lse[stage][lane] = st0.x;
-        ctl->neg_lse[stage][lane + 32] = st1.x;
-        ctl->delta[stage][lane] = st0.y;
-        ctl->delta[stage][lane + 32] = st1.y;
+        ctl->neg_lse[stage][lane] = BF16 ? st0.x : st0.x + (float)kPShift;
+        ctl->neg_lse[stage][lane + 32] = BF16 ? st1.x : st1.x + (float)kPShift;
+        ctl->neg_delta[stage][lane] = -st0.y;
+        ctl->neg_delta[stage][lane + 32] = -st1.y;
       }
       unsigned long long gone;                       // rows to clear
       if (KV) {
@@ -318,11 +388,12 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     };
 
     while (ok) {
-      const long long idx = next_idx;
-      if (idx >= P.total_items) {
-        publish(-1, 0, 0, 0, 0, 0, 0);
+      long long idx = next_idx;
+      if (idx >= total_items) {
+        publish(-1, 0, 0, 0, 0, 0, 0, 0, 0);
         break;
       }
+      if (REDO) idx = (KV ? P.sp.redo_k : P.sp.redo_q)[idx];
       if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
       next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
       if (KV) {
@@ -373,7 +444,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) n_tiles += __shfl_xor_sync(0xffffffffu, n_tiles, d);
-        publish(n_tiles, k_begin + k0, min(P.m_rows, k_end - k0), hk, k0, k_len, off);
+        publish(n_tiles, k_begin + k0, min(P.m_rows, k_end - k0), hk, k0, k_len, off, q_begin, idx);
         if (!ok || n_tiles == 0) continue;
         load_stationary(k_begin + k0, hk);
         for (int base = i_min; base < nqb && ok; base += 32) {
@@ -398,7 +469,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const int hsub = rem / P.tiles_per_qblock, qt = rem % P.tiles_per_qblock;
         const int tok0 = rec.q_begin + qt * P.tt, head0 = rec.hk * p.group + hsub * P.gp;
         if (tok0 >= rec.q_end) continue;
-        publish(rec.n_tiles, tok0, rec.q_end, head0, rec.q_in0 + qt * P.tt, rec.k_len, rec.off);
+        publish(rec.n_tiles, tok0, rec.q_end, head0, rec.q_in0 + qt * P.tt, rec.k_len, rec.off, rec.k_begin, idx);
         if (!ok || rec.n_tiles <= 0) continue;
         load_stationary(tok0, head0);
         const bool csr = p.csr_ptr != nullptr;
@@ -537,7 +608,6 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // =============================== elementwise + epilogue ===============================
     const int wg = warp >> 2, row = tid & 127;
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    const float factor = BF16 ? 1.f : fp16_grad_factor(P.head, p.headdim);
     const float scale_log2 = P.scale_log2;
     const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
     int I = 0, Iq = 0, T = 0, stage = 0;
@@ -555,17 +625,37 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       const bool valid = KV ? row < end : tok < end;
       const int hq = KV ? 0 : head + (row & (P.gp - 1));
       const int key = pos0 + row;
-      float neg_lse = -INFINITY, delta = 0.f;
+      float neg_lse = -INFINITY, neg_delta = 0.f;
       bool no_keys = false;                        // dQ: the row's log-sum-exp says that it saw no key
       int limit_row = k_len - 1;
       if (!KV) {
         if (valid && n_tiles > 0) {
-          const float2 st = P.stats[(long long)tok * p.nhead_q + hq];
+          const float2 st = P.sp.stats[(long long)tok * p.nhead_q + hq];
           neg_lse = st.x;
-          delta = st.y;
+          neg_delta = -st.y;
           no_keys = neg_lse == -INFINITY;
         }
         if (p.causal) limit_row = min(limit_row, pos0 + (row >> P.gp_shift) + off);
+      }
+      // fp16: P is formed as 2^p_exp P (2^kPShift of it by the loader), dS as 2^ds_exp dS; the largest |P| and |dS| so scaled
+      const long long kv_row = (long long)tok * p.nhead_k + head, q_row = (long long)tok * p.nhead_q + hq;
+      int p_exp = 0, ds_exp = 0, seen = 0;             // dQ: keys that the row has seen
+      float top_p = 0.f, top_ds = 0.f;
+      uint64_t p_exp2 = 0ull, ds_mul2 = 0ull;
+      if (!BF16) {
+        p_exp = KV ? kPShift : 0;
+        if (valid && n_tiles > 0) {
+          ds_exp = KV ? ds_exponent(__uint_as_float(P.sp.max_do[(long long)sl->first * p.nhead_k + head]) *
+                                    __uint_as_float(P.sp.max_v[(long long)(row0 - pos0) * p.nhead_k + head]))
+                      : ds_exponent(P.sp.norm_do[q_row] * __uint_as_float(P.sp.max_v[(long long)sl->first * p.nhead_k + hq / p.group]));
+          if (REDO) {
+            const int top = KV ? P.sp.top_k[kv_row] : P.sp.top_q[q_row];
+            if (KV) p_exp = min(p_exp + redo_exponent(top & 255), 110);
+            ds_exp = max(min(ds_exp + redo_exponent(top >> 8), 120), -120);
+          }
+        }
+        if (KV && REDO) p_exp2 = pack_f32x2((float)(p_exp - kPShift), (float)(p_exp - kPShift));
+        ds_mul2 = pack_f32x2(pow2(ds_exp - p_exp), pow2(ds_exp - p_exp));
       }
       for (int t = 0; t < n_tiles && ok; ++t, ++T) {
         if ((T & 1) == wg) {
@@ -585,6 +675,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           } else {
             const int k0 = *(volatile int*)&ctl->info0[stage], k_end = *(volatile int*)&ctl->info1[stage];
             hi_col = min(limit_row, k_end - 1) - k0;
+            if (!BF16 && !REDO) seen += max(min(hi_col + 1, 64), 0);
           }
           const bool edge = KV ? lo_col > 0 : hi_col < nt - 1;
           tmem_wait_ld();
@@ -603,11 +694,17 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 const int c = 16 * j + i;
                 float4 nl = make_float4(neg_lse, neg_lse, neg_lse, neg_lse);
                 if (KV) nl = nl4[c >> 2];
+                uint64_t nl01 = pack_f32x2(nl.x, nl.y), nl23 = pack_f32x2(nl.z, nl.w);
+                if (KV && REDO) {
+                  nl01 = add_f32x2(nl01, p_exp2);
+                  nl23 = add_f32x2(nl23, p_exp2);
+                }
                 float x0, x1, x2, x3;
-                unpack_f32x2(fma_f32x2(pack_b32x2(r[c], r[c + 1]), scale2, pack_f32x2(nl.x, nl.y)), x0, x1);
-                unpack_f32x2(fma_f32x2(pack_b32x2(r[c + 2], r[c + 3]), scale2, pack_f32x2(nl.z, nl.w)), x2, x3);
+                unpack_f32x2(fma_f32x2(pack_b32x2(r[c], r[c + 1]), scale2, nl01), x0, x1);
+                unpack_f32x2(fma_f32x2(pack_b32x2(r[c + 2], r[c + 3]), scale2, nl23), x2, x3);
                 x0 = ex2_approx(x0); x1 = ex2_approx(x1); x2 = ex2_approx(x2); x3 = ex2_approx(x3);
                 if (KV) {
+                  if (!BF16 && !REDO) top_p = max3_abs(max3_abs(top_p, x0, x1), x2, x3);
                   split2<BF16>(x0, x1, hi[i >> 1], lo[i >> 1]);
                   split2<BF16>(x2, x3, hi[(i >> 1) + 1], lo[(i >> 1) + 1]);
                 }
@@ -633,7 +730,7 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           for (int j = 0; j < 4; ++j)
             if (nt > 16 * j) tmem_ld16(tS + 64 + 16 * j, *reinterpret_cast<uint32_t(*)[16]>(&g[16 * j]));
           tmem_wait_ld();
-          const float4* dl4 = reinterpret_cast<const float4*>(ctl->delta[stage]);
+          const float4* dl4 = reinterpret_cast<const float4*>(ctl->neg_delta[stage]);
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             if (nt > 16 * j) {
@@ -641,16 +738,19 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
               for (int i = 0; i < 16; i += 4) {
                 const int c = 16 * j + i;
-                float4 dl = make_float4(delta, delta, delta, delta);
+                float4 dl = make_float4(neg_delta, neg_delta, neg_delta, neg_delta);
                 if (KV) dl = dl4[c >> 2];
-                const float d[4] = {dl.x, dl.y, dl.z, dl.w};
-                float x[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float pr = __uint_as_float(r[c + e]);
-                  x[e] = pr * (__uint_as_float(g[c + e]) - d[e]);
-                  if (!BF16) x[e] *= factor;
+                uint64_t d01 = pack_f32x2(dl.x, dl.y), d23 = pack_f32x2(dl.z, dl.w);
+                d01 = mul_f32x2(pack_b32x2(r[c], r[c + 1]), add_f32x2(pack_b32x2(g[c], g[c + 1]), d01));
+                d23 = mul_f32x2(pack_b32x2(r[c + 2], r[c + 3]), add_f32x2(pack_b32x2(g[c + 2], g[c + 3]), d23));
+                if (!BF16) {
+                  d01 = mul_f32x2(d01, ds_mul2);
+                  d23 = mul_f32x2(d23, ds_mul2);
                 }
+                float x[4];
+                unpack_f32x2(d01, x[0], x[1]);
+                unpack_f32x2(d23, x[2], x[3]);
+                if (!BF16 && !REDO) top_ds = max3_abs(max3_abs(top_ds, x[0], x[1]), x[2], x[3]);
                 split2<BF16>(x[0], x[1], hi[i >> 1], lo[i >> 1]);
                 split2<BF16>(x[2], x[3], hi[(i >> 1) + 1], lo[(i >> 1) + 1]);
               }
@@ -670,12 +770,33 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       if (!ok) break;
 
+      if (!BF16 && !REDO && n_tiles > 0) {
+        // The rows' largest values, from both warpgroups; items with a row out of range go on the redo list (once).
+        int tp = KV ? exponent_of(top_p) : min(seen, 127), ts = exponent_of(top_ds);
+        if (wg == 1) {
+          ctl->top[Iq & 1][row] = (uint16_t)(tp | ts << 8);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_of(smem_u32(ctl->top_ready), Iq));
+        } else {
+          ok = warp_wait(bar_of(smem_u32(ctl->top_ready), Iq), par_of(Iq), abort_flag, budget);
+          if (!ok) break;
+          const int other = *(volatile uint16_t*)&ctl->top[Iq & 1][row];
+          tp = KV ? max(tp, other & 255) : tp + (other & 255);
+          ts = max(ts, other >> 8);
+          if (valid) (KV ? P.sp.top_k[kv_row] : P.sp.top_q[q_row]) = (uint16_t)(tp | ts << 8);
+          const int low = top_low(n_tiles);
+          // (the dS of a row that sees a single key is what the rounding of two equal numbers leaves: small by right)
+          const bool again = __any_sync(0xffffffffu, valid && (KV ? out_of_range(tp, low) || out_of_range(ts, low) : tp > 1 && out_of_range(ts, low)));
+          if (again && lane == 0 && atomicMax(&ctl->redo_mark, Iq + 1) < Iq + 1)
+            (KV ? P.sp.redo_k : P.sp.redo_q)[atomicAdd(&P.sp.head->redo_count[KV ? 1 : 0], 1ull)] = sl->index;
+        }
+      }
+
       // ---- epilogue: KV: warpgroup 0 writes dV, 1 writes dK; dQ: each writes half of the columns
       constexpr int NC = KV ? D : D / 2;
       const int c_base = KV ? 0 : wg * NC;
-      OutT* const orow = KV ? (wg == 0 ? out0 : out1) + ((long long)tok * p.nhead_k + head) * p.headdim
-                            : out0 + ((long long)tok * p.nhead_q + hq) * p.headdim;
-      const float mul = KV && wg == 0 ? 1.f : p.scale / factor;
+      OutT* const orow = KV ? (wg == 0 ? out0 : out1) + kv_row * p.headdim : out0 + q_row * p.headdim;
+      const float mul = KV && wg == 0 ? (BF16 ? 1.f : pow2(-p_exp)) : (BF16 ? p.scale : p.scale * pow2(-ds_exp));
       if (n_tiles > 0) {
         ok = warp_wait(b_acc_full, (uint32_t)Iq & 1u, abort_flag, budget);
         if (!ok) break;
@@ -726,26 +847,71 @@ bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   }
   if (tid == 0 && ctl->abort_flag) {
     atomicExch(&P.ws.status[0], HBSA_STATUS_WAIT_LIMIT);
-    P.ws.status[3] = (int)blockIdx.x;
+    P.ws.status[3] = (int)block;
   }
 }
 
-// {-lse * log2 e, delta = rowsum(dO * O)} of every (token, q-head) row; with fp16 also max|dO| and max|V|.  16 lanes per row, 16
-// bytes per lane; bound by the read of O and dO.  Rows of q / k outside every sample get zero gradients here.
+template <int D, bool BF16, bool KV>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_x,
+                 const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ BwdParams P) {
+  bwd_body<D, BF16, KV, false>(tm_a, tm_b, tm_x, tm_y, P, blockIdx.x, gridDim.x);
+}
+// Both redo lists in one launch (usually empty ones, so what counts is one launch less): the first half of the CTAs takes dQ's.
+template <int D>
+__global__ void __launch_bounds__(kBwdThreads, 1)
+bwd_redo_kernel(const __grid_constant__ BwdMaps q, const __grid_constant__ BwdMaps kv, const __grid_constant__ BwdParams Pq,
+                const __grid_constant__ BwdParams Pkv) {
+  const unsigned half = gridDim.x / 2;
+  if (blockIdx.x < half) bwd_body<D, false, false, true>(q.a, q.b, q.x, q.y, Pq, blockIdx.x, half);
+  else bwd_body<D, false, true, true>(kv.a, kv.b, kv.x, kv.y, Pkv, blockIdx.x - half, half);
+}
+
+// Raises one slot to the largest finite x it is given, with an atomic per run of the same slot; non-negative floats order like their bits.
+struct MaxRun {
+  unsigned int* slot = nullptr;
+  float top = 0.f;
+  __device__ __forceinline__ void flush() const {
+    if (slot != nullptr && top > 0.f) atomicMax(slot, __float_as_uint(top));
+  }
+  __device__ __forceinline__ void take(unsigned int* s, float x) {
+    if (s != slot) {
+      flush();
+      slot = s;
+      top = 0.f;
+    }
+    if (x < INFINITY) top = fmaxf(top, x);
+  }
+};
+// First token of the sample that holds token `tok`; [lo, hi) is the sample found last.
+__device__ __forceinline__ int first_token(const int32_t* __restrict__ cu, int batch, int tok, int& lo, int& hi) {
+  if (tok < lo || tok >= hi) {
+    const int b = sample_of_block(cu, batch, tok);
+    lo = cu[b];
+    hi = cu[b + 1];
+  }
+  return lo;
+}
+
+// {-lse * log2 e, delta = rowsum(dO * O)} of every (token, q-head) row; with fp16 also the norms of the rows of dO, and the
+// maxima of those of dO and V over every sample and kv-head (rows that see no key and rows with Inf or NaN left out).  16 lanes per row, 16 bytes per lane; bound by the read of O and dO.
+// Rows of q / k outside every sample get zero gradients here.
 template <bool BF16>
 __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams P, const uint16_t* __restrict__ o, long long o0, long long o1,
                                                        const uint16_t* __restrict__ d_o, long long g0, long long g1,
                                                        const uint16_t* __restrict__ v, long long v0, long long v1,
-                                                       const float* __restrict__ lse, float2* __restrict__ stats, uint16_t* dq, uint16_t* dk, uint16_t* dv) {
+                                                       const float* __restrict__ lse, uint16_t* dq, uint16_t* dk, uint16_t* dv) {
   const Problem& p = P.p;
   const int chunk = threadIdx.x & 15, n_chunk = p.headdim >> 3;
-  const long long first = (long long)blockIdx.x * 16 + (threadIdx.x >> 4), step = (long long)gridDim.x * 16;
-  const long long rows = (long long)P.total_q * p.nhead_q;
-  float am = 0.f, vm = 0.f;
+  const long long step = (long long)gridDim.x * 16;
+  const long long rows = (long long)P.total_q * p.nhead_q, k_rows = (long long)P.total_k * p.nhead_k;
   const int q_lo = p.cu_q[0], q_hi = p.cu_q[p.batch], k_lo = p.cu_k[0], k_hi = p.cu_k[p.batch];
-  for (long long base = (long long)blockIdx.x * 16; base < rows; base += step) {      // uniform per block: the shuffles need whole warps
+  MaxRun run;
+  int lo = 0, hi = 0;
+  // uniform per block: the shuffles need whole warps
+  for (long long base = (long long)blockIdx.x * 16; base < rows; base += step) {
     const long long row = base + (threadIdx.x >> 4);
-    float acc = 0.f;
+    float acc = 0.f, sq = 0.f;
     const long long tok = row / p.nhead_q, h = row % p.nhead_q;
     if (row < rows && chunk < n_chunk) {
       const uint4 a = *reinterpret_cast<const uint4*>(o + tok * o0 + h * o1 + chunk * 8);
@@ -757,48 +923,58 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(BwdParams P, const uint16
         unpack16<BF16>(wa[i], x0, x1);
         unpack16<BF16>(wb[i], y0, y1);
         acc = fmaf(x0, y0, fmaf(x1, y1, acc));
-        if (!BF16) am = fmaxf(am, fmaxf(fabsf(y0), fabsf(y1)));
+        if (!BF16) sq = fmaf(y0, y0, fmaf(y1, y1, sq));
       }
     }
 #pragma unroll
-    for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    for (int s = 8; s > 0; s >>= 1) {
+      acc += __shfl_xor_sync(0xffffffffu, acc, s);
+      if (!BF16) sq += __shfl_xor_sync(0xffffffffu, sq, s);
+    }
     if (row < rows) {
+      const bool outside = tok < q_lo || tok >= q_hi;
       if (chunk == 0) {
         const float l = lse[row];
-        stats[row] = fabsf(l) < INFINITY ? make_float2(-l * kLog2e, acc) : make_float2(-INFINITY, 0.f);
+        const bool live = fabsf(l) < INFINITY;
+        P.sp.stats[row] = live ? make_float2(-l * kLog2e, acc) : make_float2(-INFINITY, 0.f);
+        if (!BF16) {
+          const float norm = sqrtf(sq);
+          P.sp.norm_do[row] = norm;
+          if (!outside && live) run.take(P.sp.max_do + (long long)first_token(p.cu_q, p.batch, (int)tok, lo, hi) * p.nhead_k + h / p.group, norm);
+        }
       }
-      if ((tok < q_lo || tok >= q_hi) && chunk < n_chunk) *reinterpret_cast<uint4*>(dq + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
+      if (outside && chunk < n_chunk) *reinterpret_cast<uint4*>(dq + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
     }
   }
-  const long long k_rows = (long long)P.total_k * p.nhead_k;
-  for (long long row = first; row < k_rows; row += step) {
+  lo = hi = 0;
+  for (long long base = (long long)blockIdx.x * 16; base < k_rows; base += step) {
+    const long long row = base + (threadIdx.x >> 4);
     const long long tok = row / p.nhead_k, h = row % p.nhead_k;
-    if (chunk < n_chunk && (tok < k_lo || tok >= k_hi)) {
+    const bool outside = tok < k_lo || tok >= k_hi;
+    if (row < k_rows && chunk < n_chunk && outside) {
       *reinterpret_cast<uint4*>(dk + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
       *reinterpret_cast<uint4*>(dv + row * p.headdim + chunk * 8) = make_uint4(0, 0, 0, 0);
     }
-    if (!BF16 && chunk < n_chunk) {
-      const uint4 a = *reinterpret_cast<const uint4*>(v + tok * v0 + h * v1 + chunk * 8);
-      const uint32_t wa[4] = {a.x, a.y, a.z, a.w};
+    if (!BF16) {
+      float sq = 0.f;
+      if (row < k_rows && chunk < n_chunk) {
+        const uint4 a = *reinterpret_cast<const uint4*>(v + tok * v0 + h * v1 + chunk * 8);
+        const uint32_t wa[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float x0, x1;
-        unpack16<BF16>(wa[i], x0, x1);
-        vm = fmaxf(vm, fmaxf(fabsf(x0), fabsf(x1)));
+        for (int i = 0; i < 4; ++i) {
+          float x0, x1;
+          unpack16<BF16>(wa[i], x0, x1);
+          sq = fmaf(x0, x0, fmaf(x1, x1, sq));
+        }
+      }
+#pragma unroll
+      for (int s = 8; s > 0; s >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, s);
+      if (row < k_rows && chunk == 0) {
+        if (!outside) run.take(P.sp.max_v + (long long)first_token(p.cu_k, p.batch, (int)tok, lo, hi) * p.nhead_k + h, sqrtf(sq));
       }
     }
   }
-  if (!BF16) {                                       // maxima of non-negative floats order like their bits
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-      am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, s));
-      vm = fmaxf(vm, __shfl_xor_sync(0xffffffffu, vm, s));
-    }
-    if ((threadIdx.x & 31) == 0) {
-      atomicMax(&P.head->amax_do, __float_as_uint(am));
-      atomicMax(&P.head->amax_v, __float_as_uint(vm));
-    }
-  }
+  if (!BF16) run.flush();
 }
 
 // q-heads packed into a tile of at most `rows` rows: the largest power of two that divides the group
@@ -818,23 +994,34 @@ int even_tile(int rows) {
   return ((rows + n - 1) / n + 15) / 16 * 16;
 }
 
+template <int D> constexpr size_t bwd_smem() { return 4u * 128u * D * 2u + 2u * kBwdStages * kBwdTile * D * 2u + sizeof(BwdControl); }
+static_assert(bwd_smem<128>() <= 227u * 1024u, "shared memory of one CTA");
+
 template <int D, bool BF16, bool KV>
-cudaError_t launch_one(const CUtensorMap& a, const CUtensorMap& b, const CUtensorMap& x, const CUtensorMap& y, const BwdParams& P, cudaStream_t stream) {
-  constexpr size_t smem = 4u * 128u * D * 2u + 2u * kBwdStages * kBwdTile * D * 2u + sizeof(BwdControl);
-  static_assert(smem <= 227u * 1024u, "shared memory of one CTA");
+cudaError_t launch_one(const BwdMaps& m, const BwdParams& P, cudaStream_t stream) {
   static SmemOptIn opt_in;
-  cudaError_t e = opt_in.once(reinterpret_cast<const void*>(bwd_sm100_kernel<D, BF16, KV>), (int)smem);
+  cudaError_t e = opt_in.once(reinterpret_cast<const void*>(bwd_sm100_kernel<D, BF16, KV>), (int)bwd_smem<D>());
   if (e != cudaSuccess) return e;
   const long long resident = sm100_sm_count();
   const unsigned grid = (unsigned)(P.total_items < resident ? P.total_items : resident);
-  bwd_sm100_kernel<D, BF16, KV><<<grid, kBwdThreads, smem, stream>>>(a, b, x, y, P);
+  bwd_sm100_kernel<D, BF16, KV><<<grid, kBwdThreads, bwd_smem<D>(), stream>>>(m.a, m.b, m.x, m.y, P);
+  return cudaGetLastError();
+}
+template <int D>
+cudaError_t launch_redo(const BwdMaps (&m)[2], const BwdParams (&P)[2], cudaStream_t stream) {
+  static SmemOptIn opt_in;
+  cudaError_t e = opt_in.once(reinterpret_cast<const void*>(bwd_redo_kernel<D>), (int)bwd_smem<D>());
+  if (e != cudaSuccess) return e;
+  bwd_redo_kernel<D><<<2 * sm100_sm_count(), kBwdThreads, bwd_smem<D>(), stream>>>(m[0], m[1], P[0], P[1]);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t backward_sm100_workspace_bytes(long long total_q, int nhead_q) {
-  return kBwdHeaderBytes + (size_t)(total_q * nhead_q) * sizeof(float2);
+size_t backward_sm100_workspace_bytes(long long total_q, long long total_k, int nhead_q, int nhead_k) {
+  BwdSpace s;
+  size_t zeroed;
+  return carve_space(nullptr, total_q, total_k, nhead_q, nhead_k, &s, &zeroed);
 }
 
 const char* backward_sm100_ineligible_reason(const hbsa_backward_args& b, float scale) {
@@ -856,17 +1043,18 @@ int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_back
   EncodeTiledFn fn = sm100_encode_fn();
   if (!fn) { *err_text = "cuTensorMapEncodeTiled is not available from the CUDA driver"; return HBSA_ERR_DRIVER; }
   const bool bf16 = a.dtype == HBSA_DTYPE_BF16;
-  BwdParams P = {};
+  BwdParams both[2] = {};                          // dQ, dK/dV
+  BwdMaps maps[2];
+  BwdParams& P = both[0];
   P.p = p;
   P.ws = ws;
-  P.head = static_cast<BwdHeader*>(b.grad_workspace);
-  float2* stats = reinterpret_cast<float2*>(static_cast<char*>(b.grad_workspace) + kBwdHeaderBytes);
-  P.stats = stats;
+  size_t zeroed;
+  carve_space(static_cast<char*>(b.grad_workspace), a.total_q, a.total_k, a.nhead_q, a.nhead_k, &P.sp, &zeroed);
   P.total_q = a.total_q;
   P.total_k = a.total_k;
   P.scale_log2 = p.scale * kLog2e;
   P.wait_budget = sm100_wait_budget();
-  cudaError_t e = cudaMemsetAsync(P.head, 0, sizeof(BwdHeader), stream);
+  cudaError_t e = cudaMemsetAsync(P.sp.head, 0, bf16 ? sizeof(BwdHeader) : zeroed, stream);
   if (e != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
   {
     const long long rows = (long long)a.total_q * a.nhead_q;
@@ -874,11 +1062,13 @@ int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_back
     const unsigned grid = (unsigned)(blocks < most ? blocks : most);
     const uint16_t *o = static_cast<const uint16_t*>(a.o), *d_o = static_cast<const uint16_t*>(b.d_o), *v = static_cast<const uint16_t*>(a.v);
     uint16_t *dq = static_cast<uint16_t*>(b.dq), *dk = static_cast<uint16_t*>(b.dk), *dv = static_cast<uint16_t*>(b.dv);
-    if (bf16) bwd_prep_kernel<true><<<grid, 256, 0, stream>>>(P, o, a.o_stride[0], a.o_stride[1], d_o, b.do_stride[0], b.do_stride[1], v, a.v_stride[0], a.v_stride[1], a.lse, stats, dq, dk, dv);
-    else bwd_prep_kernel<false><<<grid, 256, 0, stream>>>(P, o, a.o_stride[0], a.o_stride[1], d_o, b.do_stride[0], b.do_stride[1], v, a.v_stride[0], a.v_stride[1], a.lse, stats, dq, dk, dv);
+    if (bf16) bwd_prep_kernel<true><<<grid, 256, 0, stream>>>(P, o, a.o_stride[0], a.o_stride[1], d_o, b.do_stride[0], b.do_stride[1], v, a.v_stride[0], a.v_stride[1], a.lse, dq, dk, dv);
+    else bwd_prep_kernel<false><<<grid, 256, 0, stream>>>(P, o, a.o_stride[0], a.o_stride[1], d_o, b.do_stride[0], b.do_stride[1], v, a.v_stride[0], a.v_stride[1], a.lse, dq, dk, dv);
     if ((e = cudaGetLastError()) != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
   }
+  both[1] = both[0];
   for (int kv = 0; kv < 2; ++kv) {
+    BwdParams& P = both[kv];
     if (kv) {
       P.gp = pack_heads(p.group, kBwdTile);
       P.tt = even_tile(p.qbs * P.gp) / P.gp;        // tokens x heads of a q-block, split evenly
@@ -909,10 +1099,15 @@ int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_back
       *err_text = "cuTensorMapEncodeTiled rejected a q/k/v/d_o layout";
       return HBSA_ERR_UNSUPPORTED;
     }
-#define HBSA_LAUNCH_BWD(D_, BF_) (kv ? launch_one<D_, BF_, true>(k, v, q, g, P, stream) : launch_one<D_, BF_, false>(q, g, k, v, P, stream))
+    maps[kv] = kv ? BwdMaps{k, v, q, g} : BwdMaps{q, g, k, v};
+#define HBSA_LAUNCH_BWD(D_, BF_) (kv ? launch_one<D_, BF_, true>(maps[1], P, stream) : launch_one<D_, BF_, false>(maps[0], P, stream))
     if (p.headdim <= 64) e = bf16 ? HBSA_LAUNCH_BWD(64, true) : HBSA_LAUNCH_BWD(64, false);
     else e = bf16 ? HBSA_LAUNCH_BWD(128, true) : HBSA_LAUNCH_BWD(128, false);
 #undef HBSA_LAUNCH_BWD
+    if (e != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
+  }
+  if (!bf16) {
+    e = p.headdim <= 64 ? launch_redo<64>(maps, both, stream) : launch_redo<128>(maps, both, stream);
     if (e != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
   }
   return 0;

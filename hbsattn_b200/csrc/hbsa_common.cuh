@@ -189,7 +189,7 @@ cudaError_t launch_forward_generic(const Problem& p, const Workspace& ws, const 
 size_t backward_workspace_bytes(long long total_q, long long total_k, int nhead_q, int nhead_k, int headdim);
 cudaError_t launch_backward_generic(const Problem& p, const Workspace& ws, const hbsa_backward_args& b, cudaStream_t stream);
 // Backward on the tensor cores (bf16 / fp16, head dimensions up to 128); same conventions as the forward's functions below.
-size_t backward_sm100_workspace_bytes(long long total_q, int nhead_q);
+size_t backward_sm100_workspace_bytes(long long total_q, long long total_k, int nhead_q, int nhead_k);
 const char* backward_sm100_ineligible_reason(const hbsa_backward_args& b, float scale);
 // Rows of one streamed K/V tile; the schedule's tile counts must be made for it (Problem::kv_tile).
 int backward_sm100_kv_tile_rows(int kbs);
