@@ -60,10 +60,11 @@ constexpr uint32_t kBwdBuf = 128u;     // TMEM columns of one S + dP buffer
 constexpr uint32_t kBwdAcc = 256u;     // first accumulator column
 constexpr float kLog2e = 1.4426950408889634f;
 
-// First words of the gradient workspace: work cursors of the launches (dQ, dK/dV, and the two that do items again), and the number of
-// items that have to be done again (dQ, dK/dV).
+// First words of the gradient workspace: work cursors of dQ, dK/dV and of the items that are done again of each, the CTAs that have
+// left each of them, and the number of items that have to be done again (dQ, dK/dV).
 struct BwdHeader {
   unsigned long long cursor[4];
+  unsigned int left[4];
   unsigned long long redo_count[2];
 };
 
@@ -109,6 +110,7 @@ struct BwdParams {
   long long total_items;
   float scale_log2;
   long long wait_budget;
+  int debug_stall;             // debugging aid: the loader publishes nothing, every wait runs out
 };
 
 struct BwdMaps { CUtensorMap a, b, x, y; };      // stationary pair, streamed pair
@@ -135,6 +137,7 @@ struct __align__(16) BwdControl {
   unsigned long long ragged_full;             // the copies of a tile with rows to clear (see zero_rows)
   uint32_t tmem_base;
   int abort_flag;
+  int fill;                                   // the launch gave up and this is its last CTA: the outputs become NaN
   int redo_mark;                              // fp16: 1 + the last item that was put on the redo list
   uint16_t top[2][128];                       // fp16: exponents of the rows' largest |P| (dQ: keys seen) and |dS| in the tiles of warps 4-7
   int info0[kBwdStages], info1[kBwdStages];   // KV: key limit of the tile's first token; dQ: first key, one past the last key
@@ -228,12 +231,16 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
 
   const long long total_items = REDO ? (long long)P.sp.head->redo_count[KV ? 1 : 0] : P.total_items;
   if (REDO && total_items == 0) return;
-  if (P.ws.status[0] != HBSA_STATUS_OK) {       // inconsistent block counts: zero gradients
+  auto fill_outputs = [&](float x, unsigned part, unsigned parts) {
     const long long n = KV ? (long long)P.total_k * p.nhead_k * p.headdim : (long long)P.total_q * p.nhead_q * p.headdim;
-    for (long long i = (long long)block * kBwdThreads + tid; i < n; i += (long long)blocks * kBwdThreads) {
-      out0[i] = OutT(0.f);
-      if (KV) out1[i] = OutT(0.f);
+    for (long long i = (long long)part * kBwdThreads + tid; i < n; i += (long long)parts * kBwdThreads) {
+      out0[i] = OutT(x);
+      if (KV) out1[i] = OutT(x);
     }
+  };
+  const int status = *(volatile int32_t*)&P.ws.status[0];
+  if (status == HBSA_STATUS_BLOCK_COUNT_MISMATCH) {       // zero gradients
+    fill_outputs(0.f, block, blocks);
     return;
   }
 
@@ -243,6 +250,21 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
   BwdControl* const ctl = reinterpret_cast<BwdControl*>(smem + 4 * STAT + 2 * kBwdStages * STRM);
   volatile int* const abort_flag = &ctl->abort_flag;
   const long long budget = P.wait_budget;
+  // Last thing every CTA does.  A launch that gave up (or found that the one before had) owes outputs: its last CTA, when all
+  // others have written theirs, fills them with NaN, so that nobody takes them for gradients.
+  auto leave = [&]() {
+    if (tid == 0) {
+      __threadfence();
+      const bool last = atomicAdd(&P.sp.head->left[(KV ? 1 : 0) + (REDO ? 2 : 0)], 1u) == blocks - 1u;
+      ctl->fill = last && *(volatile int32_t*)&P.ws.status[0] == HBSA_STATUS_WAIT_LIMIT;
+    }
+    __syncthreads();
+    if (ctl->fill) fill_outputs(NAN, 0, 1);
+  };
+  if (__syncthreads_or(status != HBSA_STATUS_OK)) {      // (a CTA of the same launch may set it at any time)
+    leave();
+    return;
+  }
   const uint32_t b_item_full = smem_u32(ctl->item_full), b_item_done = smem_u32(ctl->item_done);
   const uint32_t b_stat_full = smem_u32(ctl->stat_full), b_stat_free = smem_u32(ctl->stat_free);
   const uint32_t b_strm_full = smem_u32(ctl->strm_full), b_strm_free = smem_u32(ctl->strm_free);
@@ -298,7 +320,7 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
     int I = 0, Iq = 0, T = 0, stage = 0;
     uint32_t stage_par = 1u;                       // parity of "stage free" for the current round (first round: free)
     uint32_t ragged_par = 0u;                      // parity of the next tile with rows to clear
-    bool ok = *abort_flag == 0;
+    bool ok = *abort_flag == 0 && P.debug_stall == 0;
     long long next_idx = 0;
     if (lane == 0) next_idx = (long long)atomicAdd(cursor, 1ull);
     next_idx = __shfl_sync(0xffffffffu, next_idx, 0);
@@ -849,6 +871,7 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
     atomicExch(&P.ws.status[0], HBSA_STATUS_WAIT_LIMIT);
     P.ws.status[3] = (int)block;
   }
+  leave();
 }
 
 template <int D, bool BF16, bool KV>
@@ -1054,6 +1077,7 @@ int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_back
   P.total_k = a.total_k;
   P.scale_log2 = p.scale * kLog2e;
   P.wait_budget = sm100_wait_budget();
+  P.debug_stall = sm100_debug_stall();
   cudaError_t e = cudaMemsetAsync(P.sp.head, 0, bf16 ? sizeof(BwdHeader) : zeroed, stream);
   if (e != cudaSuccess) { *err_text = cudaGetErrorString(e); return (int)e; }
   {

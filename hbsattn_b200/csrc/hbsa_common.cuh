@@ -178,8 +178,8 @@ cudaError_t launch_notify(const Workspace& ws, int32_t* notify, int tag, cudaStr
 cudaError_t launch_schedule(const Problem& p, const Workspace& ws, uint8_t* decisions, cudaStream_t stream);
 // K/V tiles of the tensor-core forward: 64 rows, strung together from pieces of 16 (blocks of 64 n rows: the same thing).
 constexpr int kFwdTileRows = 64, kFwdUnitRows = 16;
-// Debugging aid: clock budget of every wait inside the tensor-core kernel (<= 0: the default), and a mode in
-// which its producer warp publishes nothing, so that every other wait of the kernel runs out.
+// Debugging aid: clock budget of every wait inside the tensor-core kernels (<= 0: the default), and a mode in
+// which their producer warps publish nothing, so that every other wait of the kernel runs out.
 void sm100_set_wait_budget(long long clocks, int stall_producer);
 // Debugging aid: clock64 stamps of the first CTA's pipeline events go to this device buffer (NULL: off).
 void sm100_set_trace(long long* device_buffer);

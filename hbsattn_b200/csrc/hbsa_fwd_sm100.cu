@@ -999,6 +999,7 @@ int sm100_sm_count() {
 }
 
 long long sm100_wait_budget() { return g_wait_budget; }
+int sm100_debug_stall() { return g_debug_stall; }
 void sm100_set_wait_budget(long long clocks, int stall_producer) {
   g_wait_budget = clocks > 0 ? clocks : 4000000000ll;
   g_debug_stall = stall_producer ? 1 : 0;

@@ -37,5 +37,6 @@ bool sm100_encode_map(EncodeTiledFn fn, CUtensorMap* map, bool bf16, const void*
                       long long s_tok, long long s_head, int box_heads, int box_tokens);
 int sm100_sm_count();
 long long sm100_wait_budget();
+int sm100_debug_stall();
 
 }  // namespace hbsa

@@ -207,7 +207,8 @@ def HBSAttention(*args):
 def attention_backward(q, k, v, out, lse, d_out, cu_q_seqlens, cu_k_seqlens, block_mask, q_block_size, k_block_size, causal,
                        softmax_scale=None, num_q_block=None, num_k_block=None):
     """Gradients of ``HBSAttention`` with respect to q, k and v, given the forward's output and ``lse``
-    (``HBSAttention_with_lse``): returns ``(dq, dk, dv)`` in the dtype and shapes of q, k, v."""
+    (``HBSAttention_with_lse``): returns ``(dq, dk, dv)`` in the dtype and shapes of q, k, v.  The call does not wait for
+    the device; should the kernels give up there, the gradients are NaN and ``last_status()`` says why."""
     assert lse is not None and lse.dtype == torch.float32 and lse.shape == (q.shape[0], q.shape[1]), "lse must be float32 [total_q, nhead_q]"
     assert d_out.shape == q.shape, "the output gradient must have the shape of q"
     cu_q32, cu_k32 = _prepare(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask)

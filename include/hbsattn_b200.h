@@ -195,7 +195,8 @@ int hbsa_block_decisions(const hbsa_forward_args* args, uint8_t* decisions, int3
  *   grad_workspace   >= hbsa_backward_workspace_bytes(...) bytes of device memory, 256-byte aligned
  * The tcgen05 backward runs bf16/fp16 problems the forward's tcgen05 kernel takes, up to headdim 128 (d_o, dq, dk, dv with
  * 16-byte aligned rows); CUDA-core kernels with fp32 accumulators in grad_workspace run the rest (headdim <= 256).  fwd.impl
- * forces one of the two as in the forward.  Rows that saw no key get zero gradients.
+ * forces one of the two as in the forward.  Rows that saw no key get zero gradients.  The tcgen05 kernels give up
+ * when a wait inside them runs out: the status word says HBSA_STATUS_WAIT_LIMIT then, and every gradient of a launch that did is NaN.
  */
 typedef struct hbsa_backward_args {
   size_t struct_bytes;            /* sizeof(hbsa_backward_args) of the caller */

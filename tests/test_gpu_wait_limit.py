@@ -36,3 +36,31 @@ def test_wait_limit_is_reported_and_the_gpu_stays_usable():
                           pr["qbs"], pr["kbs"], pr["causal"], None)
     st = error_stats(gold, out)
     assert st["max_abs"] <= 2e-2 and st["mean_abs"] <= 1e-3, st
+
+
+@pytest.mark.parametrize("dtype,d", [(torch.bfloat16, 128), (torch.float16, 64)])
+def test_backward_that_gives_up_returns_nan(dtype, d):
+    import hbsattn_b200 as hb
+    from hbsattn_b200 import _lib
+    lib = _lib.load()
+    pr = make_problem(42, [256, 384], [256, 384], 4, 2, d, 128, 128, True, dtype, 0.6, "diag")
+    rest = (pr["cu_q"], pr["cu_k"], pr["mask"], pr["qbs"], pr["kbs"], pr["causal"])
+    out, lse = hb.HBSAttention_with_lse(pr["q"], pr["k"], pr["v"], *rest)
+    d_out = torch.ones_like(out)
+
+    def run():
+        return hb.attention_backward(pr["q"], pr["k"], pr["v"], out, lse, d_out, *rest)
+    before = run()
+    assert hb.last_status()[0] == 0
+    try:
+        lib.hbsa_debug_set_wait_budget(2_000_000, 1)
+        grads = run()
+        assert hb.last_status()[0] == _lib.HBSA_STATUS_WAIT_LIMIT
+        for g in grads:
+            assert torch.isnan(g).all()
+    finally:
+        lib.hbsa_debug_set_wait_budget(0, 0)
+    after = run()
+    assert hb.last_status()[0] == 0
+    for a, b in zip(before, after):
+        assert torch.equal(a, b)
