@@ -306,7 +306,8 @@ PyObject* py_backward(PyObject*, PyObject* const* o, Py_ssize_t n) {
   if (!out || !lse || !g || c.k->size(0) == 0 || out->sizes() != c.q->sizes() || g->sizes() != c.q->sizes()) Py_RETURN_NONE;
   if (out->scalar_type() != c.q->scalar_type() || g->scalar_type() != c.q->scalar_type()) Py_RETURN_NONE;
   if (lse->scalar_type() != at::kFloat || !lse->is_contiguous() || lse->dim() != 2 || lse->size(0) != c.q->size(0) || lse->size(1) != c.q->size(1)) Py_RETURN_NONE;
-  if (!g->is_contiguous()) Py_RETURN_NONE;
+  const int impl = selected_impl();
+  if (!g->is_contiguous() || impl < 0) Py_RETURN_NONE;
   c10::cuda::CUDAGuard guard(c.device());
   at::Tensor dq = c.empty(c.q->sizes(), c.q->scalar_type()), dk = c.empty(c.k->sizes(), c.q->scalar_type()), dv = c.empty(c.k->sizes(), c.q->scalar_type());
   at::Tensor ws = c.workspace();
@@ -314,7 +315,7 @@ PyObject* py_backward(PyObject*, PyObject* const* o, Py_ssize_t n) {
   at::Tensor gws = c.empty({bytes}, at::kByte);
   hbsa_backward_args b;
   std::memset(&b, 0, sizeof(b));
-  c.fill(HBSA_IMPL_AUTO, *out, ws, lse);
+  c.fill(impl == HBSA_IMPL_GENERIC ? HBSA_IMPL_GENERIC : HBSA_IMPL_AUTO, *out, ws, lse);
   b.struct_bytes = sizeof(b);
   b.fwd = c.a;
   b.d_o = g->data_ptr();

@@ -22,7 +22,8 @@ _host = _lib.load_host(_state)      # native path of the plain calls; every func
 
 
 def set_kernel_family(name: str) -> None:
-    """``'auto'`` (default), ``'sm100'`` (tcgen05 kernel, error if ineligible) or ``'generic'``."""
+    """``'auto'`` (default), ``'sm100'`` (tcgen05 kernel, error if ineligible) or ``'generic'``.  Gradients: ``'generic'`` selects
+    the CUDA-core backward too; with the other two the tensor-core backward runs what it takes and the CUDA-core one the rest."""
     if name not in _IMPLS:
         raise ValueError(f"Invalid kernel family: {name}")
     _state["impl"] = name
@@ -233,8 +234,9 @@ def attention_backward(q, k, v, out, lse, d_out, cu_q_seqlens, cu_k_seqlens, blo
         ws = alloc_workspace(k.shape[1], nqb, nkb, cu_q32.numel() - 1, dev)
         b = _lib.BackwardArgs()
         b.struct_bytes = ctypes.sizeof(_lib.BackwardArgs)
+        impl = _lib.HBSA_IMPL_GENERIC if _IMPLS[_state["impl"]] == _lib.HBSA_IMPL_GENERIC else _lib.HBSA_IMPL_AUTO
         b.fwd = make_args(q, k, v, out, cu_q32, cu_k32, block_mask, q_block_size, k_block_size, causal, softmax_scale, nqb, nkb, ws,
-                          _lib.HBSA_IMPL_AUTO, lse=lse.contiguous())
+                          impl, lse=lse.contiguous())
         b.d_o = d_out.data_ptr()
         for i in range(3):
             b.do_stride[i] = d_out.stride(i)
