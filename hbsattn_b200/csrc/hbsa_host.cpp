@@ -212,7 +212,11 @@ bool run_forward(Call& c, int impl, bool validate, const at::Tensor& out, const 
   return true;
 }
 
-bool tracked(const at::Tensor* t) { return t->unsafeGetTensorImpl()->autograd_meta() != nullptr; }
+// Whether autograd may want to hear of a call with this input: backward mode while gradients are recorded, forward mode always.
+bool tracked(const at::Tensor* t) {
+  if (t->unsafeGetTensorImpl()->autograd_meta() == nullptr) return false;
+  return c10::GradMode::is_enabled() || t->_fw_grad(0).defined();
+}
 bool modes_active() { return c10::impl::TorchDispatchModeTLS::any_modes_set(); }
 
 // attention(q, k, v, cu_q, cu_k, block_mask, q_block_size, k_block_size, causal, softmax_scale[, tile_mode[, 8 tables]]) -> out
@@ -221,7 +225,7 @@ PyObject* py_attention(PyObject*, PyObject* const* o, Py_ssize_t n) {
   if (n < 10 || n > 19 || modes_active()) Py_RETURN_NONE;
   Call c;
   if (!c.tensors(o) || !c.mask || !c.options(o + 6)) Py_RETURN_NONE;
-  if (c10::GradMode::is_enabled() && (tracked(c.q) || tracked(c.k) || tracked(c.v))) Py_RETURN_NONE;
+  if (tracked(c.q) || tracked(c.k) || tracked(c.v)) Py_RETURN_NONE;
   if (n > 10) {
     if (!PyUnicode_Check(o[10])) Py_RETURN_NONE;
     if (PyUnicode_CompareWithASCIIString(o[10], "auto") != 0) {
