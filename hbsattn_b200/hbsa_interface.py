@@ -213,6 +213,7 @@ def attention_backward(q, k, v, out, lse, d_out, cu_q_seqlens, cu_k_seqlens, blo
     assert lse is not None and lse.dtype == torch.float32 and lse.shape == (q.shape[0], q.shape[1]), "lse must be float32 [total_q, nhead_q]"
     assert d_out.shape == q.shape, "the output gradient must have the shape of q"
     cu_q32, cu_k32 = _prepare(q, k, v, cu_q_seqlens, cu_k_seqlens, block_mask)
+    lse = lse.contiguous()                           # lives until the launch: the call is given addresses
     if d_out.dtype != q.dtype:
         d_out = d_out.to(q.dtype)
     if d_out.stride(2) != 1 or any(n <= 0 or n % 8 for n in d_out.stride()[:2]):
@@ -236,7 +237,7 @@ def attention_backward(q, k, v, out, lse, d_out, cu_q_seqlens, cu_k_seqlens, blo
         b.struct_bytes = ctypes.sizeof(_lib.BackwardArgs)
         impl = _lib.HBSA_IMPL_GENERIC if _IMPLS[_state["impl"]] == _lib.HBSA_IMPL_GENERIC else _lib.HBSA_IMPL_AUTO
         b.fwd = make_args(q, k, v, out, cu_q32, cu_k32, block_mask, q_block_size, k_block_size, causal, softmax_scale, nqb, nkb, ws,
-                          impl, lse=lse.contiguous())
+                          impl, lse=lse)
         b.d_o = d_out.data_ptr()
         for i in range(3):
             b.do_stride[i] = d_out.stride(i)

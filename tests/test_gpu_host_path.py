@@ -23,3 +23,20 @@ def test_forward_mode_is_refused_whatever_the_grad_mode(which, grad_mode):
         t[which] = forward_ad.make_dual(t[which], torch.ones_like(t[which]))
         with pytest.raises((NotImplementedError, RuntimeError)):
             hb.HBSAttention(t["q"], t["k"], t["v"], pr["cu_q"], pr["cu_k"], pr["mask"], 64, 64, True, None)
+
+
+@pytest.mark.parametrize("d", [64, 18])
+def test_backward_takes_an_lse_of_any_strides(d):
+    import hbsattn_b200 as hb
+    pr = make_problem(92, [100, 60], [100, 60], 2, 1, d, 64, 64, True, torch.bfloat16 if d == 64 else torch.float32, 0.7, "diag")
+    rest = (pr["cu_q"], pr["cu_k"], pr["mask"], 64, 64, True)
+    out, lse = hb.HBSAttention_with_lse(pr["q"], pr["k"], pr["v"], *rest)
+    d_out = torch.ones_like(out)
+    want = hb.attention_backward(pr["q"], pr["k"], pr["v"], out, lse, d_out, *rest)
+    turned = lse.t().contiguous().t()                # the same values, heads first in memory
+    assert not turned.is_contiguous()
+    torch.cuda.empty_cache()                         # small blocks come one behind the other out of one segment
+    for _ in range(3):
+        got = hb.attention_backward(pr["q"], pr["k"], pr["v"], out, turned, d_out, *rest)
+        for a, b in zip(got, want):
+            assert (a.float() - b.float()).abs().max().item() <= 1e-4 * b.float().abs().max().item()      # fp32: atomics in any order
