@@ -360,6 +360,11 @@ PyObject* py_calculate_blocks(PyObject*, PyObject* const* o, Py_ssize_t n) {
   const int batch = (int)cu->size(0) - 1;
   at::Tensor first = empty(batch + 1), cu_block = empty(kGuess + 1), to_batch = empty(kGuess);
   void* const stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+  // sizes and storage: a table that is saved takes its own bytes along, not those of the guess
+  auto cut = [](at::Tensor& t, int64_t size) {
+    t.unsafeGetTensorImpl()->set_sizes_contiguous({size});
+    t.unsafeGetTensorImpl()->unsafe_storage().set_nbytes((size_t)size * sizeof(int32_t));
+  };
   auto at_i32 = [](const at::Tensor& t) { return static_cast<int32_t*>(t.data_ptr()); };
   int32_t num = 0;
   int rc;
@@ -371,8 +376,8 @@ PyObject* py_calculate_blocks(PyObject*, PyObject* const* o, Py_ssize_t n) {
     to_batch = empty(num);
     rc = lib.blocks(at_i32(*cu), batch, (int)bs, num, at_i32(cu_block), at_i32(to_batch), at_i32(first), stream);
   } else if (rc == 0) {
-    cu_block.unsafeGetTensorImpl()->set_sizes_contiguous({num + 1});
-    to_batch.unsafeGetTensorImpl()->set_sizes_contiguous({num});
+    cut(cu_block, num + 1);
+    cut(to_batch, num);
   }
   if (rc != 0) {
     fail("hbsa_calculate_blocks", rc);

@@ -40,3 +40,16 @@ def test_backward_takes_an_lse_of_any_strides(d):
         got = hb.attention_backward(pr["q"], pr["k"], pr["v"], out, turned, d_out, *rest)
         for a, b in zip(got, want):
             assert (a.float() - b.float()).abs().max().item() <= 1e-4 * b.float().abs().max().item()      # fp32: atomics in any order
+
+
+@pytest.mark.parametrize("lens,block", [([1], 16), ([30, 500, 0, 7], 64), ([70000], 16)])
+def test_block_tables_own_their_bytes_only(lens, block, tmp_path):
+    import hbsattn_b200 as hb
+    cu = torch.tensor([0, *torch.tensor(lens).cumsum(0).tolist()], dtype=torch.int32, device="cuda")
+    num, *tables = hb.calculate_blocks(cu, block)
+    assert num == sum(-(-n // block) for n in lens)
+    for t, size in zip(tables, (num + 1, num, len(lens) + 1)):
+        assert t.numel() == size and t.untyped_storage().nbytes() == 4 * size
+    torch.save(tables, tmp_path / "tables.pt")
+    for a, b in zip(tables, torch.load(tmp_path / "tables.pt")):
+        assert torch.equal(a, b)
