@@ -71,10 +71,25 @@ def build(force: bool = False, verbose: bool = False, strict: bool = False) -> s
     return out
 
 
+def host_tag() -> str:
+    """What the host extension is tied to beside its sources: the torch and the Python it was compiled against."""
+    import torch
+    return f"torch {torch.__version__}, {sys.implementation.cache_tag}"
+
+
+def host_is_stale(path: str = HOST_PATH) -> bool:
+    if not os.path.exists(path):
+        return True
+    deps = [HOST_SOURCE, os.path.join(PKG_DIR, "..", "include", "hbsattn_b200.h"), os.path.abspath(__file__)]
+    if any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps):
+        return True
+    with open(path, "rb") as f:
+        return f"[{host_tag()}]".encode() not in f.read()
+
+
 def build_host(force: bool = False) -> str:
     """Compile csrc/hbsa_host.cpp into hbsattn_b200/_host.so; returns the path."""
-    deps = [HOST_SOURCE, os.path.join(PKG_DIR, "..", "include", "hbsattn_b200.h"), os.path.abspath(__file__)]
-    if not force and os.path.exists(HOST_PATH) and all(os.path.getmtime(d) <= os.path.getmtime(HOST_PATH) for d in deps):
+    if not force and not host_is_stale():
         return HOST_PATH
     import sysconfig
 
@@ -84,7 +99,8 @@ def build_host(force: bool = False) -> str:
     include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     libs = ["torch_python", "torch", "torch_cpu", "torch_cuda", "c10", "c10_cuda"]
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-o", HOST_PATH, HOST_SOURCE, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-o", HOST_PATH, HOST_SOURCE, f'-DHBSA_HOST_TAG="[{host_tag()}]"',
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     cmd += [f"-I{d}" for d in include] + [f"-L{os.path.join(root, 'lib')}"] + [f"-l{n}" for n in libs]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:

@@ -21,6 +21,9 @@
 
 #include "../../include/hbsattn_b200.h"
 
+// The torch and the Python of this build; build.py looks for it in the file.
+extern "C" __attribute__((used, visibility("default"))) const char hbsa_host_tag[] = HBSA_HOST_TAG;
+
 namespace {
 
 // Entry points of the C ABI library the package has loaded (HBSATTN_B200_LIBRARY may select another build of it).
