@@ -21,7 +21,7 @@
 // every row of the stationary tile (a key in dK/dV, a row of q in dQ; a row of an accumulator can be scaled back exactly):
 //   first launch   2^15 P;  dS by 2^13 / (|dO row| max|V|) (dQ) or 2^13 / (max|dO| max|V|) (dK/dV), which keeps it below 2^15.
 //                  The largest |P| and |dS| of every row are kept track of on the way.
-//   second launch  items in which a row's largest value stayed below 2^-9 sqrt(tiles) (keys that share their queries with an attention sink,
+//   second launch  items in which a row's largest value stayed below 2^-10 sqrt(tiles) (keys that share their queries with an attention sink,
 //                  rows whose dO is far below their neighbours') or went above 2^16 are done again with powers of two that
 //                  bring every row's largest value to 2^14.  What is lost then is 2^-39 of it: less than the fp32 sums lose.
 // The norms and maxima are those of the sample and kv-head alone: a gradient does not depend on the rest of the batch.
@@ -105,6 +105,7 @@ struct BwdParams {
   int gp, gp_shift, n_head_sub;      // q-heads packed into one tile of q rows, tiles of heads per group
   int tt;                      // tokens per tile of q rows
   int nt;                      // rows of a streamed tile (multiple of 16)
+  int piece;                   // rows of the pieces that a tile with a block end in it is loaded in
   int m_rows, n_msub;          // KV: keys of one stationary tile, tiles per k-block
   int tiles_per_qblock, items_per_row;  // dQ: as in the forward
   long long total_items;
@@ -113,7 +114,7 @@ struct BwdParams {
   int debug_stall;             // debugging aid: the loader publishes nothing, every wait runs out
 };
 
-struct BwdMaps { CUtensorMap a, b, x, y; };      // stationary pair, streamed pair
+struct BwdMaps { CUtensorMap a, b, x, y, xp, yp; };      // stationary pair, streamed pair, streamed pair in pieces
 
 struct BwdItem {
   int n_tiles;                 // < 0: no more work
@@ -164,6 +165,9 @@ template <bool BF16> __device__ __forceinline__ void split2(float x0, float x1, 
   lo = pack2<BF16>(l0, l1);
 }
 
+// The lowest n (0 .. 64) bits.
+__device__ __forceinline__ unsigned long long first_bits(int n) { return n >= 64 ? ~0ull : (1ull << n) - 1ull; }
+
 __device__ __forceinline__ float pow2(int e) { return __int_as_float((max(min(e, 127), -126) + 127) << 23); }
 __device__ __forceinline__ int exponent_of(float x) { return (int)((__float_as_uint(x) >> 23) & 255u); }     // biased; 255: Inf or NaN
 __device__ __forceinline__ float max3_abs(float a, float b, float c) {
@@ -175,9 +179,9 @@ __device__ __forceinline__ float max3_abs(float a, float b, float c) {
 constexpr int kPShift = 15;          // fp16: P enters its products as 2^15 P
 constexpr int kTopHigh = 127 + 16, kTopGoal = 127 + 14;
 // The smallest exponent of a row's largest value that will do.  Every value of the row is off by at most 2^-25, evenly spread (2^-26.8
-// in the mean), so a sum over n tiles of 64 by 2^-23.8 sqrt(n): 2^-14 or less of the largest value from 2^-9 sqrt(n) on, a quarter
-// of what the rounding of the fp16 result loses, and that only where one value stands alone among very small ones.
-__device__ __forceinline__ int top_low(int n_tiles) { return 127 - 9 + (32 - __clz(n_tiles)) / 2; }
+// in the mean), so a sum over n tiles of 64 by 2^-23.8 sqrt(n): 2^-13 or less of the largest value from 2^-10 sqrt(n) on, no more
+// than the rounding of the fp16 result loses, and that only where one value stands alone among very small ones.
+__device__ __forceinline__ int top_low(int n_tiles) { return 127 - 10 + (32 - __clz(n_tiles)) / 2; }
 // fp16: exponent that keeps |dP - delta|, at most 2 * bound, below 2^15
 __device__ __forceinline__ int ds_exponent(float bound) {
   const int e = exponent_of(bound);
@@ -189,10 +193,15 @@ __device__ __forceinline__ int redo_exponent(int top) { return top > 0 && top < 
 
 // Streamed rows that take part in no pair: past the end of the q-block or k-block (they hold whatever follows in the packed
 // tensor: the next block or sample, or memory behind the last one) and rows of q that see no key.  Masking gives them a P of zero, but
-// 0 x NaN and 0 x Inf would still come out of dP and of the accumulating products.  So the loader clears them once the tile has
-// landed and hands the tile over afterwards; every use of them is then 0 x 0.  A row is 128 bytes per 64-dim panel, whatever the swizzle.
+// 0 x NaN and 0 x Inf would still come out of dP and of the accumulating products, so they have to be zeros in shared memory.
+//   * Block ends that fall on a piece (16 rows, or the heads of a token where those are more): the tile is loaded in pieces, those
+//     past the end from beyond the tensor, where TMA delivers zeros.  All block ends inside a sample are of this kind.
+//   * Otherwise (ends of samples, rows without keys): the loader clears the rows once the tile has landed and hands the tile over
+//     afterwards.  (Going on to the next tile meanwhile cost more in every tile than it saved in these: up to 5 %.)
 // Isolation is by block: elements that a causal mask cuts out of an active pair are multiplied by an exact zero.
-// (Clearing by the elementwise warps between the first and second products, with selects on S and dP, made the hot loop 6 % slower.)
+// A training step of 4 samples, bf16, d = 64, tiles that keep the neighbours' rows / all such tiles cleared by the loader / as here:
+// 4096 tokens, 128x80 blocks 829 / 936 / 827 us; 300 tokens, 80x48 blocks (a ragged end in most items) 631 / 738 / 660 us.  Clearing by
+// the elementwise warps, with selects on S and dP, made every tile 6 % slower.
 template <int D>
 __device__ __forceinline__ void zero_rows(uint32_t tile, uint32_t y_off, uint32_t panel_bytes, unsigned long long gone, int lane) {
   constexpr int CHUNKS = D / 8;                  // 16-byte pieces of a row
@@ -218,7 +227,7 @@ __device__ __forceinline__ void issue_ts(uint32_t acc, uint32_t a_tmem, uint64_t
 // `block` of `blocks`: the CTA's place among those of the launch that do this half.
 template <int D, bool BF16, bool KV, bool REDO>
 __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensorMap& tm_b, const CUtensorMap& tm_x, const CUtensorMap& tm_y,
-                                         const BwdParams& P, unsigned block, unsigned blocks) {
+                                         const CUtensorMap& tm_xp, const CUtensorMap& tm_yp, const BwdParams& P, unsigned block, unsigned blocks) {
   // a, b: stationary pair (K, V or Q, dO); x, y: streamed pair (Q, dO or K, V)
   using namespace ptx;
   constexpr int PANELS = D / 64;
@@ -229,6 +238,7 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
   OutT* const out1 = static_cast<OutT*>(P.out1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+  // tm_xp, tm_yp: the streamed pair in pieces
   const long long total_items = REDO ? (long long)P.sp.head->redo_count[KV ? 1 : 0] : P.total_items;
   if (REDO && total_items == 0) return;
   auto fill_outputs = [&](float x, unsigned part, unsigned parts) {
@@ -361,6 +371,21 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
         if ((lane >> P.gp_shift) < valid && lane < nt) st0 = P.sp.stats[(long long)(row0 + (lane >> P.gp_shift)) * p.nhead_q + head0 + (lane & h)];
         if ((c1 >> P.gp_shift) < valid && c1 < nt) st1 = P.sp.stats[(long long)(row0 + (c1 >> P.gp_shift)) * p.nhead_q + head0 + (c1 & h)];
       }
+      // what the tile needs is settled before the wait: the loader is on the critical path behind it
+      const int rows = KV ? min(valid << P.gp_shift, nt) : min(valid, nt);      // of the tile that are the block's
+      unsigned long long gone = 0ull;
+      bool late = false;                             // handed over only when rows have been cleared
+      if (KV) {
+        const uint32_t g0 = __ballot_sync(0xffffffffu, lane < nt && st0.x == -INFINITY);
+        const uint32_t g1 = __ballot_sync(0xffffffffu, lane + 32 < nt && st1.x == -INFINITY);
+        gone = (unsigned long long)g1 << 32 | g0;
+        if (gone != 0ull) late = (rows & (P.piece - 1)) != 0 || gone != (first_bits(nt) & ~first_bits(rows));
+      } else if (rows < nt) {
+        gone = first_bits(nt) & ~first_bits(rows);
+        late = (rows & (P.piece - 1)) != 0;
+      }
+      const uint32_t dst = sStrm + (uint32_t)stage * 2u * STRM;
+      const uint32_t bar = late ? smem_u32(&ctl->ragged_full) : b_strm_full + 8u * stage;
       if (T >= kBwdStages) ok = warp_wait(b_strm_free + 8u * stage, stage_par, abort_flag, budget);
       if (!ok) return;
       if (KV) {
@@ -369,32 +394,32 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
         ctl->neg_delta[stage][lane] = -st0.y;
         ctl->neg_delta[stage][lane + 32] = -st1.y;
       }
-      unsigned long long gone;                       // rows to clear
-      if (KV) {
-        const uint32_t g0 = __ballot_sync(0xffffffffu, lane < nt && st0.x == -INFINITY);
-        const uint32_t g1 = __ballot_sync(0xffffffffu, lane + 32 < nt && st1.x == -INFINITY);
-        gone = (unsigned long long)g1 << 32 | g0;
-      } else {
-        gone = valid < nt ? ((nt < 64 ? 1ull << nt : 0ull) - 1ull) & ~((1ull << valid) - 1ull) : 0ull;
-      }
-      const uint32_t dst = sStrm + (uint32_t)stage * 2u * STRM;
       __syncwarp();
       if (lane == 0) {
         ctl->info0[stage] = i0;
         ctl->info1[stage] = i1;
         __threadfence_block();
-        const uint32_t bar = gone != 0ull ? smem_u32(&ctl->ragged_full) : b_strm_full + 8u * stage;
         mbar_arrive_expect_tx(bar, 2u * (uint32_t)nt * D * 2u);
+        if (gone == 0ull || late) {
 #pragma unroll
-        for (int pn = 0; pn < PANELS; ++pn) {
-          tma_load_3d(dst + pn * strm_panel, &tm_x, bar, pn * 64, head0, row0);
-          tma_load_3d(dst + STRM + pn * strm_panel, &tm_y, bar, pn * 64, head0, row0);
+          for (int pn = 0; pn < PANELS; ++pn) {
+            tma_load_3d(dst + pn * strm_panel, &tm_x, bar, pn * 64, head0, row0);
+            tma_load_3d(dst + STRM + pn * strm_panel, &tm_y, bar, pn * 64, head0, row0);
+          }
         }
       }
-      if (gone != 0ull) {
-        ok = warp_wait(smem_u32(&ctl->ragged_full), ragged_par, abort_flag, budget);
+      if (gone != 0ull && !late) {
+        __syncwarp();
+        const int which = lane & 1, pn = (lane >> 1) % PANELS, r = lane / (2 * PANELS) * P.piece;
+        const int tok = r < rows ? row0 + (KV ? r >> P.gp_shift : r) : KV ? P.total_q : P.total_k;
+        const uint32_t to = dst + pn * strm_panel + (uint32_t)r * 128u;
+        if (r < nt && !which) tma_load_3d(to, &tm_xp, bar, pn * 64, head0, tok);
+        if (r < nt && which) tma_load_3d(to + STRM, &tm_yp, bar, pn * 64, head0, tok);
+      }
+      if (late) {
+        ok = warp_wait(bar, ragged_par, abort_flag, budget);
         if (!ok) {                                   // the copy is still in flight: bounded, like the others at the end
-          mbar_wait_clock(smem_u32(&ctl->ragged_full), ragged_par, budget >> 4);
+          mbar_wait_clock(bar, ragged_par, budget >> 4);
           return;
         }
         ragged_par ^= 1u;
@@ -876,9 +901,8 @@ __device__ __forceinline__ void bwd_body(const CUtensorMap& tm_a, const CUtensor
 
 template <int D, bool BF16, bool KV>
 __global__ void __launch_bounds__(kBwdThreads, 1)
-bwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ CUtensorMap tm_x,
-                 const __grid_constant__ CUtensorMap tm_y, const __grid_constant__ BwdParams P) {
-  bwd_body<D, BF16, KV, false>(tm_a, tm_b, tm_x, tm_y, P, blockIdx.x, gridDim.x);
+bwd_sm100_kernel(const __grid_constant__ BwdMaps m, const __grid_constant__ BwdParams P) {
+  bwd_body<D, BF16, KV, false>(m.a, m.b, m.x, m.y, m.xp, m.yp, P, blockIdx.x, gridDim.x);
 }
 // Both redo lists in one launch (usually empty ones, so what counts is one launch less): the first half of the CTAs takes dQ's.
 template <int D>
@@ -886,8 +910,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_redo_kernel(const __grid_constant__ BwdMaps q, const __grid_constant__ BwdMaps kv, const __grid_constant__ BwdParams Pq,
                 const __grid_constant__ BwdParams Pkv) {
   const unsigned half = gridDim.x / 2;
-  if (blockIdx.x < half) bwd_body<D, false, false, true>(q.a, q.b, q.x, q.y, Pq, blockIdx.x, half);
-  else bwd_body<D, false, true, true>(kv.a, kv.b, kv.x, kv.y, Pkv, blockIdx.x - half, half);
+  if (blockIdx.x < half) bwd_body<D, false, false, true>(q.a, q.b, q.x, q.y, q.xp, q.yp, Pq, blockIdx.x, half);
+  else bwd_body<D, false, true, true>(kv.a, kv.b, kv.x, kv.y, kv.xp, kv.yp, Pkv, blockIdx.x - half, half);
 }
 
 // Raises one slot to the largest finite x it is given, with an atomic per run of the same slot; non-negative floats order like their bits.
@@ -1027,7 +1051,7 @@ cudaError_t launch_one(const BwdMaps& m, const BwdParams& P, cudaStream_t stream
   if (e != cudaSuccess) return e;
   const long long resident = sm100_sm_count();
   const unsigned grid = (unsigned)(P.total_items < resident ? P.total_items : resident);
-  bwd_sm100_kernel<D, BF16, KV><<<grid, kBwdThreads, bwd_smem<D>(), stream>>>(m.a, m.b, m.x, m.y, P);
+  bwd_sm100_kernel<D, BF16, KV><<<grid, kBwdThreads, bwd_smem<D>(), stream>>>(m, P);
   return cudaGetLastError();
 }
 template <int D>
@@ -1114,16 +1138,21 @@ int launch_backward_sm100(const Problem& p, const Workspace& ws, const hbsa_back
     }
     P.gp_shift = log2_of(P.gp);
     P.n_head_sub = p.group / P.gp;
-    CUtensorMap q, g, k, v;
+    P.piece = kv && P.gp > 16 ? P.gp : 16;
+    CUtensorMap q, g, k, v, xp, yp;
     const int qh = P.gp, qt = P.tt, kt = kv ? 128 : P.nt;
-    if (!sm100_encode_map(fn, &q, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], qh, qt) ||
+    const int pieces_ok = kv ? sm100_encode_map(fn, &xp, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], qh, P.piece / qh) &&
+                               sm100_encode_map(fn, &yp, bf16, b.d_o, p.headdim, p.nhead_q, a.total_q, b.do_stride[0], b.do_stride[1], qh, P.piece / qh)
+                             : sm100_encode_map(fn, &xp, bf16, a.k, p.headdim, p.nhead_k, a.total_k, a.k_stride[0], a.k_stride[1], 1, P.piece) &&
+                               sm100_encode_map(fn, &yp, bf16, a.v, p.headdim, p.nhead_k, a.total_k, a.v_stride[0], a.v_stride[1], 1, P.piece);
+    if (!pieces_ok || !sm100_encode_map(fn, &q, bf16, a.q, p.headdim, p.nhead_q, a.total_q, a.q_stride[0], a.q_stride[1], qh, qt) ||
         !sm100_encode_map(fn, &g, bf16, b.d_o, p.headdim, p.nhead_q, a.total_q, b.do_stride[0], b.do_stride[1], qh, qt) ||
         !sm100_encode_map(fn, &k, bf16, a.k, p.headdim, p.nhead_k, a.total_k, a.k_stride[0], a.k_stride[1], 1, kt) ||
         !sm100_encode_map(fn, &v, bf16, a.v, p.headdim, p.nhead_k, a.total_k, a.v_stride[0], a.v_stride[1], 1, kt)) {
       *err_text = "cuTensorMapEncodeTiled rejected a q/k/v/d_o layout";
       return HBSA_ERR_UNSUPPORTED;
     }
-    maps[kv] = kv ? BwdMaps{k, v, q, g} : BwdMaps{q, g, k, v};
+    maps[kv] = kv ? BwdMaps{k, v, q, g, xp, yp} : BwdMaps{q, g, k, v, xp, yp};
 #define HBSA_LAUNCH_BWD(D_, BF_) (kv ? launch_one<D_, BF_, true>(maps[1], P, stream) : launch_one<D_, BF_, false>(maps[0], P, stream))
     if (p.headdim <= 64) e = bf16 ? HBSA_LAUNCH_BWD(64, true) : HBSA_LAUNCH_BWD(64, false);
     else e = bf16 ? HBSA_LAUNCH_BWD(128, true) : HBSA_LAUNCH_BWD(128, false);
