@@ -14,6 +14,8 @@ LAYOUTS = [
     (8, 2, 64, 80, 48, False),
     (3, 1, 96, 48, 144, True),
     (8, 1, 32, 16, 16, True),
+    (2, 1, 128, 80, 80, True),            # blocks that end inside a tile of their sample
+    (32, 1, 64, 16, 80, True),            # tiles of two tokens, 32 heads each
 ]
 
 
