@@ -720,7 +720,7 @@ def ours_arm(args):
             "config": {"workload": f"{args.workload}: {w['desc']}", "per_gpu": "every rank runs the whole workload with its own seed",
                        "active_block_pairs_per_gpu": active_pairs, "flop_per_step_per_gpu": flops,
                        "l2": "q+k+v+o exceed the 126 MB L2; no flush", "kernel_family": {1: "generic", 2: "sm100"}.get(family, str(family)),
-                       "step": "schedule build (3 small kernels) + attention kernel"},
+                       "step": "schedule build (1 small kernel) + attention kernel"},
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "traffic": TRAFFIC_BYTES.get(args.workload),
                          "traffic_source": "one ncu capture of this kernel on the batch-2 cut, scaled by work items" if args.workload in TRAFFIC_BYTES else None,

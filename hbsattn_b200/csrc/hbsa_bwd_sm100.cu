@@ -30,7 +30,7 @@
 // dK 1.8955e-3 -> 1.8944e-3, dV 1.6515e-3 -> 1.6515e-3.  dV of fp16 keys beside a sink (CUDA cores / P unscaled / these): sink 16
 // above, 8192 keys, dO of 256: 2.08e-4 / 0.17 / 2.09e-4; 20 above, 4096 keys, dO of 1024: 2.26e-4 / 1.0 / 2.26e-4.  Nearly flat fp16
 // rows over 16384 keys: 2.21e-4 / 3.50e-4 / 2.25e-4; what is left there comes from the length of the fp32 accumulation (2048 products
-// in a row).  The scales and the redo launch take 2 % of the ragged fp16 training step above.
+// in a row).  The scales and the redo launch take 2 to 3 % of the ragged fp16 training step above.
 //
 // 320 threads, one persistent CTA per SM (TMEM: two tile buffers of 64 S + 64 dP columns, two accumulators of 128):
 //   warps 0-3 / 4-7   elementwise work on the even / odd tiles (thread = TMEM lane), then the epilogue: dV / dK, or the two

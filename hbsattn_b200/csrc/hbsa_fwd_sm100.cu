@@ -11,7 +11,7 @@
 //    two-slot ring in shared memory and runs ahead of them.  Two CTAs per SM mean two independent
 //    items in flight, so the start and the end of one item hide behind the tiles of the other.
 //  * Only mask-active k-blocks are touched: the producer warp compacts the mask row with warp
-//    ballots and issues TMA loads of exactly those K/V tiles (64 rows each) into two-stage K
+//    ballots and issues TMA loads of exactly those K/V tiles (64 rows each) into K
 //    and V rings (the reference loops over all k-blocks of the sample and polls the mask byte,
 //    fwd_triton_fix_tile_size.py:117-124).
 //  * S = Q K^T and O += P V are tcgen05.mma instructions with fp32 accumulators in TMEM.  S is
@@ -219,7 +219,8 @@ __device__ __forceinline__ void issue_pv(uint32_t tO, const uint32_t (&pa)[4], c
 // pieces of the item's output, reading each other's parts through distributed shared memory.  No scratch in global memory, no second
 // kernel.  A CTA works on one item only (the hardware hands out the clusters), so nothing is reused and nobody leaves
 // before the closing cluster barrier.  One token on 16 contexts of 16k to 32k keys, 8 kv-heads, d = 64: 128 items left 20 SMs
-// idle and the others with one CTA each, 125 us; in parts of 2 / 4 / 8: 81 / 83 / 110 us.
+// idle and the others with one CTA each; in parts of 1 / 2 / 4 / 8, rings of four stages: 103.5 / 59.5 / 72.7 / 106.4 us (with rings of
+// two the unshared launch took 125 us).
 template <int D, bool BF16, bool TRACE, bool GATHER, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 2)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -1063,7 +1064,8 @@ int launch_forward_sm100(const Problem& p, const Workspace& ws, const hbsa_forwa
   const long long resident = (p.headdim > 128 ? 1ll : 2ll) * sm100_sm_count();
   // Too few items for the chip: 2, 4 or 8 CTAs share an item, as long as they are needed to fill it and each of them gets 24
   // tiles of the average sample (the mask, of which the host knows nothing, leaves perhaps a tenth to a third of
-  // them).  Below that the cluster's meeting costs as much as the tiles saved (samples of 16 to 500 keys in parts of 2: 54 -> 64 us).
+  // them).  The count doubles until the chip is full, so it may end above the places there are: 128 items of a decoding step go to 512
+  // CTAs on 296 places (72.7 us), where 256 would do better (59.5 us).  Below 24 tiles the cluster's meeting costs as much as the tiles saved (samples of 16 to 500 keys in parts of 2: 54 -> 64 us).
   P.split = 1;
   while (P.split < 8 && P.total_items * P.split < resident && a.total_k / kTileRows / p.batch >= kSplitTiles * 2 * P.split) P.split *= 2;
   const bool split = P.split > 1 && P.trace == nullptr;

@@ -222,10 +222,10 @@ int hbsa_select_impl(const hbsa_forward_args* args);
  * calls it. */
 int hbsa_read_status(const void* workspace, int32_t* status_out, void* stream);
 
-/* Debugging aid (process-wide, not thread-safe).  Every wait inside the tensor-core attention kernel
+/* Debugging aid (process-wide, not thread-safe).  Every wait inside the tensor-core kernels, forward and backward,
  * gives up after `clocks` ticks of the SM clock (<= 0 restores the default of about two seconds): the
  * kernel then sets HBSA_STATUS_WAIT_LIMIT, all of its warps leave, and the call returns normally.
- * With stall_producer != 0 the kernel's loader warp publishes no work at all, so that every other
+ * With stall_producer != 0 the kernels' loader warps publish no work at all, so that every other
  * wait of the kernel runs out with nothing in flight - the way the give-up path is tested.
  * Applies to launches made after the call. */
 void hbsa_debug_set_wait_budget(long long clocks, int stall_producer);
